@@ -145,11 +145,18 @@ __device__ __forceinline__ float ld_ro(const float* p) {
 }
 
 // Programmatic dependent launch: an engine kernel lets the next kernel of its
-// stream be scheduled as soon as all of its own CTAs run, and that kernel
-// builds its twiddle tables and reads its descriptors (nothing an earlier
-// kernel writes) while this one finishes, then waits for it to complete
-// before touching any plane.  The wait is the hardware's grid dependency: it
-// ends when the earlier grid has completed and its writes are visible.
+// stream be scheduled as soon as all of its own CTAs run and its own wait for
+// the previous kernel is over, and that kernel builds its twiddle tables and
+// reads its descriptors (nothing an earlier kernel writes) while this one
+// finishes, then waits for it to complete before touching any plane.  The
+// wait is the hardware's grid dependency: it ends when the earlier grid has
+// completed and its writes are visible.
+// The next kernel is let in only after the wait: let in at entry, a chain of
+// short passes piles up on the chip several kernels deep, and a kernel's CTAs
+// then fall on whichever slots come free, several of them on one SM while
+// others idle (256^2 x 4, 64 CTAs a pass: 12.3 us per iteration against 8.7
+// with at most one waiting kernel; 512^2 x 1: 15.2 against 12.8; 128 trials of
+// 512^2 unchanged).
 __device__ __forceinline__ void pdl_allow_next() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -76,7 +76,6 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
   using RG = RowGroup<N, E>;
   extern __shared__ float2 smem[];
   __shared__ __align__(16) Slot sl[3][RG::NG];
-  pdl_allow_next();
   const int tick = (a.tick_base ? *a.tick_base : 0) + a.tick_off;
   const float2* tw = stage_twiddles<N, E>(smem + SM::kTw, a.tw);  // block barrier
   float* sup_tile = reinterpret_cast<float*>(smem + SM::kSup);
@@ -91,6 +90,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
   if (i1.slot >= 0) load_slot_by<RG::GT>(&sl[1][g], &a.slots[i1.slot], gtid);
   sync();
   pdl_wait_prev();  // the planes are the previous pass's output
+  pdl_allow_next();
   bool ready = false;
   if (row_finishes(sl[0][g], tick)) {
     prefetch_row_tile<N, E>(sl[0][g], i0.block, smem, g, gtid);
@@ -145,7 +145,6 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, false)) col_pass_k
   using CS = ColSmem<N, E>;
   extern __shared__ float2 smem[];
   __shared__ __align__(16) Slot sl[3];
-  pdl_allow_next();
   const int tick = (a.tick_base ? *a.tick_base : 0) + a.tick_off;
   const float2* tw = stage_twiddles<N, E>(smem + CS::kTw, a.tw);  // block barrier
   float* mod = reinterpret_cast<float*>(smem + CS::kMod);
@@ -158,6 +157,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, false)) col_pass_k
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
   pdl_wait_prev();  // the planes (and the transposed modulus) are earlier kernels' output
+  pdl_allow_next();
   copy_col_g<N, E>(sl[0], i0.block, tick, smem);
   asm volatile("cp.async.commit_group;" ::: "memory");
   float2* pend = nullptr;  // plane whose last stage is left in the other buffer
@@ -225,7 +225,6 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   static_assert(SPLIT * CS::C == lines_per_item(N, E), "an item is SPLIT whole sub-items");
   extern __shared__ float2 smem[];
   __shared__ __align__(16) Slot sl[3];
-  pdl_allow_next();
   const int tick = (a.tick_base ? *a.tick_base : 0) + a.tick_off;
   const float2* tw = stage_twiddles<N, E>(smem + CS::kTw, a.tw);  // block barrier
   float* mod = reinterpret_cast<float*>(smem + CS::kMod);
@@ -246,6 +245,7 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
   pdl_wait_prev();  // the planes (and the transposed modulus) are earlier kernels' output
+  pdl_allow_next();
   copy_col_mod<N, E, TH>(sl[0], i0.block, tick, mod);
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (col_projects(sl[0], tick)) copy_col_tile<N, E, TH>(sl[0].g, i0.block, tile);
