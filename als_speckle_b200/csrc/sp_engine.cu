@@ -86,9 +86,9 @@ static cudaError_t pc_setup_size(int N) {
 }
 
 // Per device, per (logN, E): dynamic-smem attributes set and the resident CTAs
-// per SM of the column pass ([0]) and row pass ([1]) cached.
+// per SM of each pass kind cached.
 static std::mutex g_setup_mutex;
-static int g_occ[64][13][3][2];  // [device][log2 N][E = 8, 16, 32][pass]; 0 = not yet configured
+static int g_occ[64][13][3][kPassKinds];  // [device][log2 N][E = 8, 16, 32][kind]; 0: not yet configured
 static int g_sms[64];
 
 static cudaError_t occupancy_for(int N, int E, int* occ, int* sms) {
@@ -103,14 +103,12 @@ static cudaError_t occupancy_for(int N, int E, int* occ, int* sms) {
     if (e != cudaSuccess) return e;
   }
   if (g_occ[dev][l][k][0] == 0) {
-    int o[2] = {0, 0};
+    int o[kPassKinds] = {};
     e = pass_setup(N, E, o);
     if (e != cudaSuccess) return e;
-    g_occ[dev][l][k][0] = std::max(1, o[0]);
-    g_occ[dev][l][k][1] = std::max(1, o[1]);
+    for (int w = kPassKinds - 1; w >= 0; --w) g_occ[dev][l][k][w] = std::max(1, o[w]);
   }
-  occ[0] = g_occ[dev][l][k][0];
-  occ[1] = g_occ[dev][l][k][1];
+  for (int w = 0; w < kPassKinds; ++w) occ[w] = g_occ[dev][l][k][w];
   *sms = g_sms[dev];
   return cudaSuccess;
 }
@@ -304,6 +302,7 @@ static cudaError_t launch_transpose(const float* src, float* dst, int N, cudaStr
 // one launch target: the items of one size within one group
 struct Segment {
   int N, E, first, count, grid[2];  // grid[pass]: 0 column, 1 row
+  int kind[2];                      // pass kind launched for each
   int pc_first, pc_count, pc_grid;  // partial-coherence jobs of this size
   int pc_egrid;                     // grid of the tiled rescale kernel
   int col_ticks;                    // the column pass runs at ticks [0, col_ticks)
@@ -342,7 +341,7 @@ static int launch_segment(const Segment& sg, const Slot* slots, const Item* item
       // whose G planes the row pass wrote last (still in L2), and the next
       // row pass starts on the ones it wrote last
       PassArgs a{slots, items + sg.first, sg.count, nullptr, k, tw, which == 0 ? 1 : 0};
-      SP_CUDA_TRY(launch_pass(sg.N, sg.E, which, sg.grid[which], st, a));
+      SP_CUDA_TRY(launch_pass(sg.N, sg.E, sg.kind[which], sg.grid[which], st, a));
     }
   }
   return SP_OK;
@@ -500,9 +499,9 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       }
       const int count = (int)hi.size() - first;
       if (count == 0) continue;
-      int occ[2] = {1, 1}, sms = 1;
+      int occ[kPassKinds], sms = 1;
       SP_CUDA_TRY(occupancy_for(N, E, occ, &sms));
-      Segment sg{N, E, first, count, {1, 1}, (int)hj.size(), 0, 1, 1, 0, 0, 0};
+      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, 0};
       for (int i = gstart[g]; i < gstart[g + 1]; ++i)
         if (trials[i].n == N) sg.ticks = std::max(sg.ticks, trials[i].n_iter + 1);
       // Partially coherent slots project in their own kernels: the column
@@ -514,9 +513,10 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
         else if (trials[i].init == SP_INIT_RANDOM_PHASE) sg.col_ticks = std::max(sg.col_ticks, 1);
       }
       for (int p = 0; p < 2; ++p) {
-        int per_sm = occ[p];
+        if (use_small_ctas(N, E, count, sms)) sg.kind[p] = p == 0 ? kPassColSmall : kPassRowSmall;
+        int per_sm = occ[sg.kind[p]];
         if (opts && opts->ctas_per_sm > 0) per_sm = std::min(per_sm, (int)opts->ctas_per_sm);
-        const int units = p == 0 ? count * col_split(N, E) : count;
+        const int units = count * pass_units(N, E, sg.kind[p]);
         sg.grid[p] = std::max(1, std::min(units, sms * per_sm));
       }
       for (int i = gstart[g]; i < gstart[g + 1]; ++i) {
@@ -629,7 +629,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
     }
     GraphKey key{workspace_dev, dev, g, ticks[g], {}};
     for (const Segment& sg : segs[g])
-      key.shape.insert(key.shape.end(), {sg.N, sg.E, sg.first, sg.count, sg.grid[0], sg.grid[1],
+      key.shape.insert(key.shape.end(), {sg.N, sg.E, sg.first, sg.count, sg.grid[0], sg.grid[1], sg.kind[0], sg.kind[1],
                                          sg.pc_first, sg.pc_count, sg.pc_grid, sg.pc_egrid,
                                          std::min(sg.ticks, sg.col_ticks), sg.pc_mask, sg.ticks});
     cudaGraphExec_t exec = nullptr;

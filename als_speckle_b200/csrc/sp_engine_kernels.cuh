@@ -236,9 +236,9 @@ __device__ __forceinline__ void cp_async_rows(void* sdst, const void* gsrc, int 
 // holds the item's G rows and then serves as its exchange buffer, the other
 // receives its psi rows and, once the update has read them, the next item's
 // G rows) | twiddles | support tile (L rows of N + 16 floats).
-template <int N, int E>
+template <int N, int E, int TH = kThreads>
 struct RowSmem {
-  static constexpr int L = lines_per_item(N, E);
+  static constexpr int L = lines_per_item_t(N, E, TH);
   // row pitch of both buffers: the padded line, rounded up to an even number
   // of complex values so every row starts 16-byte aligned (cp.async)
   static constexpr int kStrip = (padk(N, pad_shift(E)) + 1) & ~1;
@@ -309,15 +309,15 @@ struct LineSync {
 // own rows (G, psi, support) and its own slot descriptor, so every wait in
 // the row pass is a warp or line barrier and the groups of a block run
 // independently of one another.
-template <int N, int E>
+template <int N, int E, int TH = kThreads>
 struct RowGroup {
   static constexpr int T = N / E;
-  static constexpr int L = lines_per_item(N, E);
+  static constexpr int L = lines_per_item_t(N, E, TH);
   static constexpr int GT = T < 32 ? 32 : T;
   static constexpr int LPG = GT / T;
   static constexpr int ROWS = LPG < L ? LPG : L;  // lines of every group that has any
   static constexpr int NG = (L + LPG - 1) / LPG;  // groups with lines
-  static_assert(NG * GT <= kThreads && NG <= 15, "row groups");
+  static_assert(NG * GT <= TH && NG <= 15, "row groups");
   using Sync = typename std::conditional<(T <= 32), WarpSync, LineSync<T>>::type;
   __device__ static Sync sync(int g) {
     if constexpr (T <= 32) return Sync{};
@@ -352,11 +352,11 @@ __device__ __forceinline__ bool row_finishes(const Slot& s, int tick) {
 }
 
 // Copy group g's G rows of a row item into its padded strips of buf.
-template <int N, int E>
+template <int N, int E, int TH>
 __device__ __forceinline__ void prefetch_row_tile(const Slot& s, int block, float2* buf, int g,
                                                   int gtid) {
-  using RG = RowGroup<N, E>;
-  constexpr int P = RowSmem<N, E>::kStrip;
+  using RG = RowGroup<N, E, TH>;
+  constexpr int P = RowSmem<N, E, TH>::kStrip;
   const int l0 = g * RG::LPG;
   cp_async_rows<RG::ROWS, N * 8, N * 8, P * 8, RG::GT>(
       buf + l0 * P, s.g + ((size_t)block * RG::L + l0) * N, gtid);
@@ -374,20 +374,20 @@ __device__ __forceinline__ void prefetch_row_tile(const Slot& s, int block, floa
 // storage); returns whether it did (with the caller's `extra` copies in the
 // same group), and the caller swaps the buffers.
 // ---------------------------------------------------------------------------
-template <int N, int E, class Extra>
+template <int N, int E, int TH, class Extra>
 __device__ __forceinline__ bool row_item(const Slot& s, int step, int block, float2* gbuf,
                                          float2* pbuf, bool ready, float* sup_tile,
                                          const Slot* nxt, int nxt_block, int tick,
                                          const float2* __restrict__ tw, int g, int gtid,
                                          Extra&& extra) {
-  using RG = RowGroup<N, E>;
+  using RG = RowGroup<N, E, TH>;
   constexpr int T = N / E;
-  constexpr int L = lines_per_item(N, E);
+  constexpr int L = lines_per_item_t(N, E, TH);
   constexpr int SH = pad_shift(E);
-  constexpr int P = RowSmem<N, E>::kStrip;
-  constexpr int SPITCH = RowSmem<N, E>::kSupPitch;
+  constexpr int P = RowSmem<N, E, TH>::kStrip;
+  constexpr int SPITCH = RowSmem<N, E, TH>::kSupPitch;
   const int tid = threadIdx.x;
-  constexpr bool kFull = (L * T == kThreads);  // every thread owns a line segment
+  constexpr bool kFull = (L * T == TH);  // every thread owns a line segment
   const int lrow = tid / T;
   const int t = tid - lrow * T;
   const bool active = kFull || lrow < L;
@@ -425,7 +425,7 @@ __device__ __forceinline__ bool row_item(const Slot& s, int step, int block, flo
   auto prefetch_next = [&]() {
     if (nxt != nullptr && alg_f != SP_DM && alg_s != SP_DM && row_finishes(*nxt, tick)) {
       sync();  // the group is done with its part of pbuf
-      prefetch_row_tile<N, E>(*nxt, nxt_block, pbuf, g, gtid);
+      prefetch_row_tile<N, E, TH>(*nxt, nxt_block, pbuf, g, gtid);
       extra();
       asm volatile("cp.async.commit_group;" ::: "memory");
       prefetched = true;

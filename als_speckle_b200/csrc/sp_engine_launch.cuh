@@ -41,6 +41,18 @@ __device__ __forceinline__ Item item_at(const PassArgs& a, int it) {
   return it < a.n_items ? a.items[a.reverse ? a.n_items - 1 - it : it] : Item{-1, 0};
 }
 
+// Kernels of TH-thread CTAs walk sub-items: an item (kThreads threads' lines)
+// is pass_split of them, and sub-item j is part j % SPLIT of item j / SPLIT.
+__host__ __device__ constexpr int pass_split(int N, int E, int TH) {
+  return lines_per_item(N, E) / lines_per_item_t(N, E, TH);
+}
+template <int SPLIT>
+__device__ __forceinline__ Item sub_item(const PassArgs& a, int j) {
+  Item i = item_at(a, j / SPLIT);
+  i.block = SPLIT * i.block + j % SPLIT;
+  return i;
+}
+
 // E = 32 keeps 64 registers of line data per thread plus the prefetched
 // psi/support: one 256-thread CTA per SM with up to 255 registers.  E = 16
 // halves that and runs two CTAs per SM.
@@ -70,10 +82,12 @@ __device__ __forceinline__ const float2* stage_twiddles(float2* tw, const float2
 // requested as soon as its psi rows of the current item have been consumed,
 // together with the descriptor of the item after that; the item list is read
 // ahead into registers.
-template <int N, int E>
-__global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_kernel(PassArgs a) {
-  using SM = RowSmem<N, E>;
-  using RG = RowGroup<N, E>;
+template <int N, int E, int TH>
+__global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
+    row_pass_kernel(PassArgs a) {
+  using SM = RowSmem<N, E, TH>;
+  using RG = RowGroup<N, E, TH>;
+  constexpr int SPLIT = pass_split(N, E, TH);
   extern __shared__ float2 smem[];
   __shared__ __align__(16) Slot sl[3][RG::NG];
   const int tick = (a.tick_base ? *a.tick_base : 0) + a.tick_off;
@@ -81,11 +95,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
   float* sup_tile = reinterpret_cast<float*>(smem + SM::kSup);
   const int g = threadIdx.x / RG::GT;
   const int gtid = threadIdx.x - g * RG::GT;
+  const int n_sub = SPLIT * a.n_items;
   int it = blockIdx.x;
-  if (g >= RG::NG || it >= a.n_items) return;  // no lines for this group, or no items
+  if (g >= RG::NG || it >= n_sub) return;  // no lines for this group, or no items
   const auto sync = RG::sync(g);
   const int G = gridDim.x;
-  Item i0 = item_at(a, it), i1 = item_at(a, it + G), i2 = item_at(a, it + 2 * G);
+  Item i0 = sub_item<SPLIT>(a, it), i1 = sub_item<SPLIT>(a, it + G), i2 = sub_item<SPLIT>(a, it + 2 * G);
   load_slot_by<RG::GT>(&sl[0][g], &a.slots[i0.slot], gtid);
   if (i1.slot >= 0) load_slot_by<RG::GT>(&sl[1][g], &a.slots[i1.slot], gtid);
   sync();
@@ -93,13 +108,13 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
   pdl_allow_next();
   bool ready = false;
   if (row_finishes(sl[0][g], tick)) {
-    prefetch_row_tile<N, E>(sl[0][g], i0.block, smem, g, gtid);
+    prefetch_row_tile<N, E, TH>(sl[0][g], i0.block, smem, g, gtid);
     asm volatile("cp.async.commit_group;" ::: "memory");
     ready = true;
   }
   int par = 0;
-  for (int k = 0; it < a.n_items; it += G, ++k) {
-    const Item i3 = item_at(a, it + 3 * G);
+  for (int k = 0; it < n_sub; it += G, ++k) {
+    const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
     sync();  // the group is done with its rows of both buffers and with item k-1's slot entry
     const Slot& s = sl[k % 3][g];
     auto copy_ring = [&]() {  // item k+2's descriptor into item k-1's entry
@@ -108,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
     const int step = tick - s.start_tick;
     bool next_ready = false;
     if (step >= 0 && step <= s.n_iter) {
-      next_ready = row_item<N, E>(s, step, i0.block, smem + par * SM::kB, smem + (par ^ 1) * SM::kB,
+      next_ready = row_item<N, E, TH>(s, step, i0.block, smem + par * SM::kB, smem + (par ^ 1) * SM::kB,
                                   ready, sup_tile, i1.slot >= 0 ? &sl[(k + 1) % 3][g] : nullptr,
                                   i1.block, tick, tw, g, gtid, copy_ring);
     }
@@ -140,49 +155,52 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, true)) row_pass_ke
 // round a ring of three (items k, k+1 and k+2, whose copy is requested during
 // item k), and the item list is read ahead into registers, so no step of the
 // loop waits on a global load.
-template <int N, int E>
-__global__ void __launch_bounds__(kThreads, min_blocks_for(E, false)) col_pass_kernel(PassArgs a) {
-  using CS = ColSmem<N, E>;
+template <int N, int E, int TH>
+__global__ void __launch_bounds__(TH, min_blocks_for(E, false) * (kThreads / TH))
+    col_pass_kernel(PassArgs a) {
+  using CS = ColSmem<N, E, TH>;
+  constexpr int SPLIT = pass_split(N, E, TH);
   extern __shared__ float2 smem[];
   __shared__ __align__(16) Slot sl[3];
   const int tick = (a.tick_base ? *a.tick_base : 0) + a.tick_off;
   const float2* tw = stage_twiddles<N, E>(smem + CS::kTw, a.tw);  // block barrier
   float* mod = reinterpret_cast<float*>(smem + CS::kMod);
+  const int n_sub = SPLIT * a.n_items;
   int it = blockIdx.x;
-  if (it >= a.n_items) return;  // the whole block leaves together
+  if (it >= n_sub) return;  // the whole block leaves together
   const int G = gridDim.x;
   // items k, k+1, k+2 held in registers; item k+3 is read during item k
-  Item i0 = item_at(a, it), i1 = item_at(a, it + G), i2 = item_at(a, it + 2 * G);
+  Item i0 = sub_item<SPLIT>(a, it), i1 = sub_item<SPLIT>(a, it + G), i2 = sub_item<SPLIT>(a, it + 2 * G);
   load_slot(&sl[0], &a.slots[i0.slot]);
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
   pdl_wait_prev();  // the planes (and the transposed modulus) are earlier kernels' output
   pdl_allow_next();
-  copy_col_g<N, E>(sl[0], i0.block, tick, smem);
+  copy_col_g<N, E, TH>(sl[0], i0.block, tick, smem);
   asm volatile("cp.async.commit_group;" ::: "memory");
   float2* pend = nullptr;  // plane whose last stage is left in the other buffer
   int pend_block = 0;
   int b = 0;
-  for (int k = 0; it < a.n_items; it += G, ++k, b ^= 1) {
-    const Item i3 = item_at(a, it + 3 * G);
+  for (int k = 0; it < n_sub; it += G, ++k, b ^= 1) {
+    const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
     cp_async_wait_all();  // this item's G tile and item k+1's slot descriptor
     __syncthreads();      // ... visible to all; the previous item is finished
     float2* other = smem + (b ^ 1) * CS::kB;
     const Slot& s = sl[k % 3];
     auto copies = [&]() {
-      copy_col_mod<N, E>(s, i0.block, tick, mod);
+      copy_col_mod<N, E, TH>(s, i0.block, tick, mod);
       asm volatile("cp.async.commit_group;" ::: "memory");
-      if (i1.slot >= 0) copy_col_g<N, E>(sl[(k + 1) % 3], i1.block, tick, other);
+      if (i1.slot >= 0) copy_col_g<N, E, TH>(sl[(k + 1) % 3], i1.block, tick, other);
       if (i2.slot >= 0) copy_slot(&sl[(k + 2) % 3], &a.slots[i2.slot]);  // item k-1's entry
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (pend)
-      col_last_stage<N, E>(pend, pend_block, other, tw, copies);
+      col_last_stage<N, E, TH>(pend, pend_block, other, tw, copies);
     else
       copies();
     pend = nullptr;
     if (col_live(s, tick)) {
-      pend = col_item<N, E>(s, tick - s.start_tick, i0.block, smem + b * CS::kB, mod, tw);
+      pend = col_item<N, E, TH>(s, tick - s.start_tick, i0.block, smem + b * CS::kB, mod, tw);
       pend_block = i0.block;
     }
     i0 = i1;
@@ -190,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks_for(E, false)) col_pass_k
     i2 = i3;
   }
   __syncthreads();
-  if (pend) col_last_stage<N, E>(pend, pend_block, smem + (b ^ 1) * CS::kB, tw, [] {});
+  if (pend) col_last_stage<N, E, TH>(pend, pend_block, smem + (b ^ 1) * CS::kB, tw, [] {});
   cp_async_wait_all();
 }
 
@@ -214,7 +232,7 @@ constexpr int kColSbThreads = 128;
 __host__ __device__ constexpr bool col_single_buffered(int N, int E) { return N == 512 && E == 32; }
 // column-pass work units per item
 __host__ __device__ constexpr int col_split(int N, int E) {
-  return col_single_buffered(N, E) ? lines_per_item(N, E) / lines_per_item_t(N, E, kColSbThreads) : 1;
+  return col_single_buffered(N, E) ? pass_split(N, E, kColSbThreads) : 1;
 }
 
 template <int N, int E>
@@ -233,14 +251,8 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   int it = blockIdx.x;
   if (it >= n_sub) return;  // the whole block leaves together
   const int G = gridDim.x;
-  auto sub_at = [&](int j) -> Item {
-    if (j >= n_sub) return Item{-1, 0};
-    Item i = item_at(a, j / SPLIT);
-    i.block = SPLIT * i.block + j % SPLIT;
-    return i;
-  };
   // sub-items k, k+1, k+2 held in registers; sub-item k+3 is read during k
-  Item i0 = sub_at(it), i1 = sub_at(it + G), i2 = sub_at(it + 2 * G);
+  Item i0 = sub_item<SPLIT>(a, it), i1 = sub_item<SPLIT>(a, it + G), i2 = sub_item<SPLIT>(a, it + 2 * G);
   load_slot(&sl[0], &a.slots[i0.slot]);
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   if (col_projects(sl[0], tick)) copy_col_tile<N, E, TH>(sl[0].g, i0.block, tile);
   asm volatile("cp.async.commit_group;" ::: "memory");
   for (int k = 0; it < n_sub; it += G, ++k) {
-    const Item i3 = sub_at(it + 3 * G);
+    const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
     cp_async_wait_all();  // this sub-item's modulus and tile, sub-item k+1's descriptor
     __syncthreads();      // ... visible to all; the previous sub-item is finished
     const Slot& s = sl[k % 3];
@@ -278,47 +290,93 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   cp_async_wait_all();
 }
 
-template <int N, int E>
-constexpr size_t col_smem_bytes() {
-  if constexpr (col_single_buffered(N, E))
-    return (size_t)ColTile<N, E, kColSbThreads>::kTotal * sizeof(float2);
-  else
-    return (size_t)ColSmem<N, E>::kTotal * sizeof(float2);
+// Lone trials and small batches: when the items of kThreads-thread CTAs are
+// too few for the chip (a 256^2 trial is 16 of them at E = 16, on 16 of 148
+// SMs), both passes run in kSmallThreads-thread CTAs on quarter items instead
+// (the same kernels, so bitwise the same results): a lone pass is bound by its
+// warps' own instruction chains, which run faster with 2 warps on an SM than
+// with 8.  Taken up to two small CTAs per SM (one at 512^2, where two of them
+// are as slow as a large one); measured, us per iteration in large / small
+// CTAs, small CTAs in brackets: 256^2 x 1 8.5 / 6.1 [64], x 2 8.6 / 7.4 [128],
+// x 4 8.7 / 8.5 [256], x 8 9.3 / 10.5 [512]; 512^2 x 1 12.8 / 11.2 [128], x 4
+// 16.1 / 17.4 [512]; 128^2 x 1 14.7 / 8.4 [8], x 36 15.5 / 12.1 [288]; 64^2 x
+// 40 11.9 / 9.4 [80].  At 1024^2 a trial is 128 items already.
+constexpr int kSmallThreads = 64;
+__host__ __device__ constexpr bool has_small_ctas(int N, int E) {
+  return N >= 64 && N <= 512 && pass_split(N, E, kSmallThreads) > 1;
 }
-template <int N, int E>
-constexpr size_t row_smem_bytes() { return (size_t)RowSmem<N, E>::kTotal * sizeof(float2); }
+
+// pass kinds: 0 column, 1 row, and the same in small CTAs
+enum { kPassCol = 0, kPassRow = 1, kPassColSmall = 2, kPassRowSmall = 3, kPassKinds = 4 };
+
+template <int N, int E, int TH>
+constexpr size_t col_smem_bytes() {
+  if constexpr (TH == kColSbThreads)
+    return (size_t)ColTile<N, E, TH>::kTotal * sizeof(float2);
+  else
+    return (size_t)ColSmem<N, E, TH>::kTotal * sizeof(float2);
+}
+template <int N, int E, int TH>
+constexpr size_t row_smem_bytes() { return (size_t)RowSmem<N, E, TH>::kTotal * sizeof(float2); }
+
+// Call f(kernel, threads, dynamic shared memory) for a pass kind of (N, E);
+// cudaErrorInvalidValue for one that is not compiled.
+template <int N, int E, class F>
+cudaError_t with_pass_kernel(int which, F&& f) {
+  if (which == kPassCol) {
+    if constexpr (col_single_buffered(N, E))
+      return f(col_pass_sb_kernel<N, E>, kColSbThreads, col_smem_bytes<N, E, kColSbThreads>());
+    else
+      return f(col_pass_kernel<N, E, kThreads>, kThreads, col_smem_bytes<N, E, kThreads>());
+  }
+  if (which == kPassRow)
+    return f(row_pass_kernel<N, E, kThreads>, kThreads, row_smem_bytes<N, E, kThreads>());
+  if constexpr (has_small_ctas(N, E)) {
+    if (which == kPassColSmall)
+      return f(col_pass_kernel<N, E, kSmallThreads>, kSmallThreads,
+               col_smem_bytes<N, E, kSmallThreads>());
+    if (which == kPassRowSmall)
+      return f(row_pass_kernel<N, E, kSmallThreads>, kSmallThreads,
+               row_smem_bytes<N, E, kSmallThreads>());
+  }
+  return cudaErrorInvalidValue;
+}
 
 template <int N, int E>
 cudaError_t launch_pass_t(int which, int grid, cudaStream_t st, const PassArgs& a) {
-  if (which == 0) {
-    if constexpr (col_single_buffered(N, E))
-      return launch_pdl(col_pass_sb_kernel<N, E>, grid, kColSbThreads, col_smem_bytes<N, E>(), st, a);
-    else
-      return launch_pdl(col_pass_kernel<N, E>, grid, kThreads, col_smem_bytes<N, E>(), st, a);
-  }
-  return launch_pdl(row_pass_kernel<N, E>, grid, kThreads, row_smem_bytes<N, E>(), st, a);
+  return with_pass_kernel<N, E>(which, [&](void (*k)(PassArgs), int threads, size_t smem) {
+    return launch_pdl(k, grid, threads, smem, st, a);
+  });
 }
 
-// occupancy[0] = resident column-pass CTAs per SM, occupancy[1] = row-pass
-// (the column pass's CTAs each take 1 / col_split(N, E) of an item)
+// occupancy[kind] = resident CTAs per SM of each pass kind (0: not compiled)
 template <int N, int E>
 cudaError_t pass_setup_t(int* occupancy) {
-  const int sc = (int)col_smem_bytes<N, E>(), sr = (int)row_smem_bytes<N, E>();
-  cudaError_t e;
-  if constexpr (col_single_buffered(N, E)) {
-    e = cudaFuncSetAttribute(col_pass_sb_kernel<N, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
+  for (int which = 0; which < kPassKinds; ++which) {
+    occupancy[which] = 0;
+    if (which >= kPassColSmall && !has_small_ctas(N, E)) continue;
+    const cudaError_t e =
+        with_pass_kernel<N, E>(which, [&](void (*k)(PassArgs), int threads, size_t smem) {
+          cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+          if (r != cudaSuccess) return r;
+          return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy[which], k, threads, smem);
+        });
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy[0], col_pass_sb_kernel<N, E>,
-                                                      kColSbThreads, sc);
-  } else {
-    e = cudaFuncSetAttribute(col_pass_kernel<N, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy[0], col_pass_kernel<N, E>, kThreads, sc);
   }
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(row_pass_kernel<N, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occupancy[1], row_pass_kernel<N, E>, kThreads, sr);
+  return cudaSuccess;
+}
+
+// Does a segment of `items` items of (N, E) run in small CTAs?
+inline bool use_small_ctas(int N, int E, int items, int sms) {
+  return has_small_ctas(N, E) && items * pass_split(N, E, kSmallThreads) <= (N <= 256 ? 2 : 1) * sms;
+}
+
+// work units of one item in each pass kind
+inline int pass_units(int N, int E, int which) {
+  if (which == kPassCol) return col_split(N, E);
+  if (which == kPassRow) return 1;
+  return pass_split(N, E, kSmallThreads);
 }
 
 // Per-size entry points (defined in sp_engine_n<N>.cu).  E is clamped to N.
