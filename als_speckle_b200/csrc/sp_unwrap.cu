@@ -73,8 +73,133 @@ __device__ void bspline3_line(const T* in, double* out, int n, long stride) {
   }
 }
 
-// Columns first (thread j walks column j: neighbouring threads touch
-// neighbouring addresses), from the float map into the FP64 coefficients.
+// Lines of kSegMin and more are prefiltered in segments of kSeg values, one
+// thread each: the recursions forget their past by |z| = 0.268 a step, so a
+// thread that starts kWarm = 32 steps before its segment (after it, for the
+// anti-causal one) from zero is off by |z|^32 = 5e-19 of the line's scale,
+// below FP64's rounding, and the exact boundary sums need 64 terms only.  One
+// thread per line (kept for short and very long lines) is a chain of 4 n
+// dependent FP64 steps on n threads: at 512 lines of 512 it took 238 us for
+// the columns and 247 us for the rows; the segments take 8 and 7 us.
+constexpr int kSeg = 16, kWarm = 32, kSegMin = 128;
+constexpr int kSegRowMax = 8192;  // longest row staged in shared memory
+
+// the causal recursion's first value of a line of n >= kSegMin samples,
+// p[0] = 6 sum_k z^k x[k] (the mirrored terms carry z^(n-1) < 1e-70)
+template <class F>
+__device__ __forceinline__ double bspline3_first(F&& x) {
+  double s = 0.0;
+#pragma unroll 16
+  for (int k = 63; k >= 0; --k) s = x(k) + kZ3 * s;
+  return kGain3 * s;
+}
+
+// Columns, thread (column j, segment): p in registers over the segment and
+// the warm-up of the way back; the map is only read and c only written, so
+// segments are independent.
+__global__ void __launch_bounds__(128) spline_cols_seg_kernel(const float* __restrict__ in,
+                                                              double* __restrict__ c, int N) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s0 = blockIdx.y * kSeg;
+  if (j >= N) return;
+  const float* x = in + j;
+  double prev = 0.0;
+  int k = s0 - kWarm;
+  if (k <= 0) {
+    prev = bspline3_first([&](int i) { return (double)x[(size_t)i * N]; });
+    k = 1;
+  }
+#pragma unroll 16
+  for (; k < s0; ++k) prev = kGain3 * (double)x[(size_t)k * N] + kZ3 * prev;
+  const double before = prev;  // p[s0 - 1]
+  double p[kSeg + kWarm];
+#pragma unroll
+  for (int i = 0; i < kSeg + kWarm; ++i) {
+    const int q = s0 + i;
+    if (q > 0 && q < N) prev = kGain3 * (double)x[(size_t)q * N] + kZ3 * prev;
+    p[i] = prev;  // (q = 0: prev is p[0] already; past the end: p[N-1])
+  }
+  double next = 0.0;
+#pragma unroll
+  for (int i = kSeg + kWarm - 1; i >= 0; --i) {
+    const int q = s0 + i;
+    if (q < N - 1) {
+      next = kZ3 * (next - p[i]);
+    } else if (q == N - 1) {  // the anti-causal boundary value
+      next = (kZ3 / (kZ3 * kZ3 - 1.0)) * (p[i] + kZ3 * (i > 0 ? p[i - 1] : before));
+    }
+    if (i < kSeg && q < N) c[(size_t)q * N + j] = next;
+  }
+}
+
+// Rows in place, one warp per row: the row and its causal values in shared
+// memory (one spare value per kSeg, so that lanes a segment apart fall on
+// different banks), segments dealt to the lanes.  A row with a value that is
+// not finite becomes NaN as a whole, as the unsegmented recursions make it
+// (unwrap_kernel does the same across rows).
+__device__ __forceinline__ int seg_pad(int k) { return k + k / kSeg; }
+__global__ void spline_rows_seg_kernel(double* __restrict__ c, int N) {
+  extern __shared__ double row_s[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = blockIdx.x * (blockDim.x >> 5) + w;
+  double* x = row_s + (size_t)w * (N + N / kSeg + 1) * 2;  // inputs, then c
+  double* p = x + (N + N / kSeg + 1);
+  if (row >= N) return;
+  double* g = c + (size_t)row * N;
+  bool bad = false;
+  for (int k = lane; k < N; k += 32) {
+    const double v = g[k];
+    bad |= !isfinite(v);
+    x[seg_pad(k)] = v;
+  }
+  if (__any_sync(0xffffffffu, bad)) {
+    for (int k = lane; k < N; k += 32) g[k] = nan("");
+    return;
+  }
+  __syncwarp();
+  const double first = bspline3_first([&](int i) { return x[seg_pad(i)]; });
+  for (int s0 = lane * kSeg; s0 < N; s0 += 32 * kSeg) {
+    double prev = 0.0;
+    int k = s0 - kWarm;
+    if (k <= 0) {
+      prev = first;
+      k = 1;
+    }
+#pragma unroll 8
+    for (; k < s0; ++k) prev = kGain3 * x[seg_pad(k)] + kZ3 * prev;
+    const int e = s0 + kSeg < N ? s0 + kSeg : N;
+    if (s0 == 0) p[0] = first;
+#pragma unroll 8
+    for (; k < e; ++k) {
+      prev = kGain3 * x[seg_pad(k)] + kZ3 * prev;
+      p[seg_pad(k)] = prev;
+    }
+  }
+  __syncwarp();
+  for (int s0 = lane * kSeg; s0 < N; s0 += 32 * kSeg) {
+    const int e = s0 + kSeg < N ? s0 + kSeg : N;
+    double next = 0.0;
+    int k = e + kWarm - 1;
+    if (k >= N - 1) {
+      next = (kZ3 / (kZ3 * kZ3 - 1.0)) * (p[seg_pad(N - 1)] + kZ3 * p[seg_pad(N - 2)]);
+      if (e == N) x[seg_pad(N - 1)] = next;
+      k = N - 2;
+    }
+#pragma unroll 8
+    for (; k >= e; --k) next = kZ3 * (next - p[seg_pad(k)]);
+#pragma unroll 8
+    for (; k >= s0; --k) {
+      next = kZ3 * (next - p[seg_pad(k)]);
+      x[seg_pad(k)] = next;
+    }
+  }
+  __syncwarp();
+  for (int k = lane; k < N; k += 32) g[k] = x[seg_pad(k)];
+}
+
+// One thread per line.  Columns first (thread j walks column j: neighbouring
+// threads touch neighbouring addresses), from the float map into the FP64
+// coefficients.
 __global__ void spline_cols_kernel(const float* __restrict__ in, double* __restrict__ c, int N) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= N) return;
@@ -129,12 +254,27 @@ __device__ __forceinline__ double bspline3_at(const double* __restrict__ c, int 
 // One block per radius r_in + blockIdx.x: the samples at the `cols` angles
 // phi_k = 2 pi k / cols (wrapping.py:46-51 order of operations), written to
 // `unwrapped` (row-major, radius by angle) if given, and their mean to `mean`.
+// A map with a value that is not finite unwraps to NaN everywhere (the
+// prefilter's recursions carry it along every line); after the segmented
+// prefilter (`rows_poisoned`) such a value shows as a row of NaN, found here
+// in the first column.
 __global__ void unwrap_kernel(const double* __restrict__ c, int N, int r_in, int cols, double cy,
-                              double cx, float* __restrict__ unwrapped, float* __restrict__ mean) {
+                              double cx, float* __restrict__ unwrapped, float* __restrict__ mean,
+                              int rows_poisoned) {
   constexpr double kPi = 3.141592653589793238462643383279502884;
   const int row = blockIdx.x;
   const double r = (double)(r_in + row);
   double part = 0.0;
+  if (rows_poisoned) {
+    bool bad = false;
+    for (int k = threadIdx.x; k < N; k += blockDim.x) bad |= !isfinite(c[(size_t)k * N]);
+    if (__syncthreads_or(bad)) {
+      for (int k = threadIdx.x; k < cols; k += blockDim.x)
+        if (unwrapped) unwrapped[(size_t)row * cols + k] = nanf("");
+      if (threadIdx.x == 0 && mean) mean[row] = nanf("");
+      return;
+    }
+  }
   for (int k = threadIdx.x; k < cols; k += blockDim.x) {
     const double phi = (double)k * 2.0 * kPi / (double)cols;
     double sn, cs;
@@ -178,12 +318,25 @@ extern "C" int sp_unwrap(const float* in_dev, int N, int r_in, int r_out, double
            cy, cx, N, N);
   cudaStream_t st = as_stream(stream);
   const int tb = 128, nb = (N + tb - 1) / tb;
-  spline_cols_kernel<<<nb, tb, 0, st>>>(in_dev, work_dev, N);
+  const bool seg = N >= kSegMin && N <= kSegRowMax;
+  if (seg)
+    spline_cols_seg_kernel<<<dim3(nb, (N + kSeg - 1) / kSeg), tb, 0, st>>>(in_dev, work_dev, N);
+  else
+    spline_cols_kernel<<<nb, tb, 0, st>>>(in_dev, work_dev, N);
   SP_CUDA_TRY(cudaGetLastError());
-  spline_rows_kernel<<<nb, tb, 0, st>>>(work_dev, N);
+  if (seg) {
+    const size_t row_bytes = (size_t)(N + N / kSeg + 1) * 2 * sizeof(double);
+    const int warps = row_bytes * 4 <= 64 * 1024 ? 4 : 1;  // rows per CTA
+    SP_CUDA_TRY(cudaFuncSetAttribute(spline_rows_seg_kernel,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(row_bytes * warps)));
+    spline_rows_seg_kernel<<<(N + warps - 1) / warps, 32 * warps, row_bytes * warps, st>>>(work_dev, N);
+  } else {
+    spline_rows_kernel<<<nb, tb, 0, st>>>(work_dev, N);
+  }
   SP_CUDA_TRY(cudaGetLastError());
   unwrap_kernel<<<r_out - r_in, 256, 0, st>>>(work_dev, N, r_in, columns, cy, cx, unwrapped_dev,
-                                               mean_dev);
+                                               mean_dev, seg ? 1 : 0);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }

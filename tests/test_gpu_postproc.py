@@ -119,3 +119,34 @@ def test_unwrap_general_grid_vs_oracle():
     want = O.unwrap(m, r_in, r_out, (cy, cx), columns=cols)
     assert np.allclose(uw.cpu().numpy(), want, rtol=1e-5, atol=1e-6)
     assert np.allclose(mean.cpu().numpy(), want.mean(axis=1), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("N", [64, 127, 128, 129, 143, 160, 513, 1000, 2500])
+def test_unwrap_segmented_prefilter_vs_oracle(N):
+    """Both prefilters (one thread per line below 128, segments from there) on
+    a white-noise map, at sizes around the switch, the segment length and the
+    rows-per-CTA switch.  The samples are float32 roundings of FP64 values
+    that agree far below a float32 ulp, so two may differ by one ulp (1.2e-7
+    relative)."""
+    import torch
+    from als_speckle_b200._lib import call, ptr, stream_ptr
+    m = np.random.default_rng(N).standard_normal((N, N)).astype(np.float32)
+    r_out, c, cols = N // 2, float(N // 2), 301
+    a = torch.from_numpy(m).cuda()
+    work = torch.empty((N, N), dtype=torch.float64, device="cuda")
+
+    def run():
+        uw = torch.empty((r_out, cols), dtype=torch.float32, device="cuda")
+        mean = torch.empty(r_out, dtype=torch.float32, device="cuda")
+        call("sp_unwrap", ptr(a), N, 0, r_out, c, c, cols, ptr(work), ptr(uw), ptr(mean), stream_ptr())
+        return uw.cpu().numpy(), mean.cpu().numpy()
+
+    uw, mean = run()
+    want = O.unwrap(m, 0, r_out, (c, c), columns=cols)
+    assert np.allclose(uw, want, rtol=2.5e-7, atol=1e-11)
+    assert np.allclose(mean, want.astype(np.float64).mean(axis=1), rtol=1e-6, atol=1e-7)
+    # a value that is not finite reaches every sample
+    for bad in (np.nan, np.inf):
+        a[N // 3, N // 5] = bad
+        uw, mean = run()
+        assert not np.isfinite(uw).any() and not np.isfinite(mean).any()
