@@ -107,6 +107,7 @@ _SIGS = {
     "sp_multiply_axis_f_f2": ([_i, _p, _p, _p, _i64, _p], _i),
     "sp_multiply_f2_f2": ([_p, _p, _p, _i64, _p], _i),
     "sp_rftf_accumulate": ([_i, _p, _p, _p, _i, _i, _p], _i),
+    "sp_rftf_frames": ([_p, _i, _i, _i, _p, _i, _p, _p, _p], _i),
     "sp_rftf_map": ([_p, _p, _i, _i, _p, _p, _p, _p], _i),
     "sp_rftf_from_error": ([_p, _p, _i64, _i, _p], _i),
     "sp_remove_hot_pixels": ([_p, _p, _i, _i, _i, _i, _f, _p], _i),

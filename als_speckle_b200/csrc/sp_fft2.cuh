@@ -79,6 +79,261 @@ __global__ void __launch_bounds__(kThreads) fft_cols_kernel(const float2* in,
   }
 }
 
+// ---------------------------------------------------------------------------
+// 2-D transforms of frames (n, rows, cols) embedded at the corner of zeroed
+// N x N planes, reduced over the frames pixel by pixel (PRTF, RFTF), without
+// making the zeros or storing the transforms: the row kernel transforms only
+// the frames' own rows, straight from the frames, and leaves them transposed,
+// so that a column is contiguous; in the column kernel every line of a CTA is
+// then a column of its own, loaded, transformed and added up in registers with
+// no barrier wider than the line.  128 frames of 180^2 at N = 512: 40 us of rows
+// (store-bound: 94 MB in 64-byte pieces), 71 us of columns (instruction issue)
+// and 12 us to add the partial sums up, against 435 us for embedding, two
+// passes over the planes and an accumulation; columns interleaved in a CTA,
+// with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 66 us, from
+// 128 us.  Radix 32 (two stages at 512) made the columns 65 us but changed the
+// transforms' rounding.
+// ---------------------------------------------------------------------------
+struct EmbedArgs {
+  const float2* src;
+  float2* dst;  // n planes of N x N: plane f, row c = column c of frame f's row transforms
+  int n, rows, cols;
+  const float2* tw;
+};
+
+constexpr int kEmbedThreads = 128;  // column kernel
+// values per thread: those of sp_fft2, so that the transforms are its bit for
+// bit (where F is nearly 0 its phasor amplifies any change of rounding), but
+// for 4096 points, which need 128 threads
+__host__ __device__ constexpr int embed_e(int N) { return N >= 4096 ? 32 : (N < 16 ? N : 16); }
+// resident CTAs per SM the kernels are compiled for
+__host__ __device__ constexpr int embed_ctas(int N) { return embed_e(N) > 16 ? 3 : 5; }
+
+// The row kernel's lines, in strips whose pitch (as the column pass's) makes
+// the transposed reads, L rows of 16 / L columns per half-warp, conflict-free.
+template <int N>
+struct EmbedRows {
+  static constexpr int E = embed_e(N), T = N / E, L = lines_per_item(N, E), SH = pad_shift(E);
+  static constexpr int P = L >= 16 ? next_congruent(padk(N, SH), 1, 2)
+                                   : next_congruent(padk(N, SH), 16 / L, 16);
+  static constexpr int kTw = L * P;
+  static constexpr int kTotal = kTw + tw_stage_total(N, E);
+};
+
+template <int T>
+struct EmbedSync {
+  using type = typename std::conditional<(T <= 32), WarpSync, LineSync<T>>::type;
+  __device__ static type make(int line) {
+    if constexpr (T <= 32) return type{};
+    else return type{1 + line};
+  }
+};
+
+template <int N>
+__global__ void __launch_bounds__(kThreads, embed_e(N) > 16 ? 1 : 3) embed_rows_kernel(EmbedArgs a) {
+  using ER = EmbedRows<N>;
+  constexpr int E = ER::E, T = ER::T, L = ER::L, SH = ER::SH;
+  extern __shared__ float2 smem[];
+  float2* tw = smem + ER::kTw;
+  build_stage_twiddles<N, E>(tw, a.tw + N);
+  __syncthreads();
+  const int lrow = threadIdx.x / T;
+  const int t = threadIdx.x - lrow * T;
+  const bool line = lrow < L;
+  const RowLayout<SH> lay{smem + (line ? lrow : 0) * ER::P};
+  const auto sync = EmbedSync<T>::make(lrow);
+  const int blocks = (a.rows + L - 1) / L;  // of one frame
+  const int64_t items = (int64_t)a.n * blocks;
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const int64_t f = it / blocks;
+    const int r0 = (int)(it - f * blocks) * L;
+    const bool mine = line && r0 + lrow < a.rows;
+    const float2* src = a.src + (f * a.rows + r0 + (mine ? lrow : 0)) * a.cols;
+    float2 v[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int c = t + i * T;
+      v[i] = (mine && c < a.cols) ? src[c] : make_float2(0.f, 0.f);
+    }
+    fft_line<N, E, -1>(v, lay, sync, line, t, tw);
+    sync();  // the line's last stage has read its strip
+    if (line) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) lay.at(t + i * T) = v[i];
+    }
+    __syncthreads();
+    const int nr = a.rows - r0 < L ? a.rows - r0 : L;
+    float2* dst = a.dst + f * N * N + r0;
+    for (int q = threadIdx.x; q < L * N; q += kThreads) {
+      const int r = q % L, c = q / L;
+      if (r < nr) dst[(size_t)c * N + r] = smem[r * ER::P + padk(c, SH)];
+    }
+    __syncthreads();  // the strips are free
+  }
+}
+
+// Columns of the transposed planes, one line of T threads each.  The work is
+// the (column group, frame) pairs, groups outermost, dealt to the CTAs in equal
+// runs of `run` pairs; a CTA adds up its frames of one group and stores the
+// sum over the lines' own rows of the first plane it read for them (each
+// thread overwrites only what it alone has read), still transposed.  So the
+// sums of group g lie in planes f with f = 0 or (g n + f) % run = 0 (see
+// for_each_sum).  `Op` maps (F, pixel) to the summand.
+__host__ __device__ constexpr int embed_group_cols(int N) {
+  return lines_per_item_t(N, embed_e(N), kEmbedThreads);
+}
+template <int N, class Op>
+__global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_kernel(EmbedArgs a, Op op,
+                                                                                  int run) {
+  constexpr int E = embed_e(N), T = N / E, L = embed_group_cols(N);
+  constexpr int SH = pad_shift(E);
+  extern __shared__ float2 smem[];
+  float2* tw = smem + L * padk(N, SH);
+  build_stage_twiddles<N, E>(tw, a.tw + N);
+  __syncthreads();
+  const int lc = threadIdx.x / T;
+  const int t = threadIdx.x - lc * T;
+  const bool active = lc < L;
+  const RowLayout<SH> lay{smem + (active ? lc : 0) * padk(N, SH)};
+  const auto sync = EmbedSync<T>::make(lc);
+  const int64_t total = (int64_t)(N / L) * a.n;
+  int64_t u = (int64_t)blockIdx.x * run;
+  const int64_t end = u + run < total ? u + run : total;
+  while (u < end) {
+    const int g = (int)(u / a.n), f0 = (int)(u - (int64_t)g * a.n);
+    const int nf = (int)(end - u < a.n - f0 ? end - u : a.n - f0);
+    const int col = g * L + (active ? lc : 0);
+    float2* p = a.dst + (size_t)f0 * N * N + (size_t)col * N + t;
+    typename Op::Acc acc[E];
+    typename Op::Pixel px[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      acc[i] = typename Op::Acc{};
+      px[i] = op.pixel((size_t)(t + i * T) * N + col);
+    }
+    for (int f = 0; f < nf; ++f) {
+      const float2* q = p + (size_t)f * N * N;
+      float2 v[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+        v[i] = (active && t + i * T < a.rows) ? __ldcg(q + i * T) : make_float2(0.f, 0.f);
+      fft_line<N, E, -1>(v, lay, sync, active, t, tw);
+      bool odd = false;
+#pragma unroll
+      for (int i = 0; i < E; ++i) odd |= !op.add(acc[i], v[i], px[i]);
+      if (odd) {
+#pragma unroll 1
+        for (int i = 0; i < E; ++i) {
+          // (register arrays take constant indexes only: pick element i)
+          float2 x = v[0];
+          typename Op::Pixel y = px[0];
+          typename Op::Acc z{};
+#pragma unroll
+          for (int k = 1; k < E; ++k)
+            if (k == i) x = v[k], y = px[k];
+          op.add_odd(z, x, y);
+#pragma unroll
+          for (int k = 0; k < E; ++k)
+            if (k == i) Op::plus(acc[k], z);
+        }
+      }
+    }
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) p[i * T] = Op::store(acc[i]);
+    }
+    u += nf;
+  }
+}
+
+// f(plane) for every plane that holds a sum of column c
+template <class F>
+__device__ __forceinline__ void for_each_sum(int c, int group_cols, int n, int run, F&& f) {
+  const int64_t base = (int64_t)(c / group_cols) * n;
+  f(0);
+  for (int k = run - (int)(base % run); k < n; k += run) f(k);
+}
+
+// F/|F| summed (phasing_prtf_accumulate2.cl:20-23); nothing where F = 0.  The
+// reciprocal square root takes one Newton step (to ~1 ulp, as hypotf and a
+// division); magnitudes whose square leaves the normal range go through hypotf.
+struct PhasorSum {
+  struct Pixel {};
+  using Acc = float2;
+  __device__ static float2 store(float2 x) { return x; }
+  __device__ static void plus(float2& a, float2 b) { a.x += b.x, a.y += b.y; }
+  __device__ Pixel pixel(size_t) const { return {}; }
+  __device__ __forceinline__ static bool plain(float p2) { return p2 > 1e-30f && p2 < 1e30f; }
+  // adds the summand unless its magnitude needs add_odd; whether it did
+  __device__ __forceinline__ bool add(float2& acc, float2 v, Pixel) const {
+    const float p2 = v.x * v.x + v.y * v.y;
+    const bool ok = plain(p2);
+    float r = ok ? rsqrtf(p2) : 0.f;
+    r = r * fmaf(-0.5f * p2 * r, r, 1.5f);
+    acc.x = ok ? fmaf(v.x, r, acc.x) : acc.x;
+    acc.y = ok ? fmaf(v.y, r, acc.y) : acc.y;
+    return ok;
+  }
+  __device__ void add_odd(float2& acc, float2 v, Pixel) const {
+    if (plain(v.x * v.x + v.y * v.y)) return;
+    const float h = hypotf(v.x, v.y);
+    if (h > 0.f) {
+      acc.x += v.x / h;
+      acc.y += v.y / h;
+    }
+  }
+};
+
+// 1/sqrt(1 + (g - |F|)^2 / g^2) summed (phasing_rftf_accumulate.cl), g the goal
+// modulus.  1/sqrt(x) by the reciprocal square root and one Newton step;
+// nothing needs a slow form (at g = 0 the quotient is infinite, or NaN for
+// F = 0 too, as in the division).
+struct RftfSum {
+  const float* goal;
+  struct Pixel {
+    float g, inv;  // g, 1/g^2
+  };
+  using Acc = float;
+  __device__ static float2 store(float x) { return make_float2(x, 0.f); }
+  __device__ static void plus(float& a, float b) { a += b; }
+  __device__ Pixel pixel(size_t k) const {
+    const float g = goal[k];
+    return {g, 1.f / (g * g)};
+  }
+  __device__ __forceinline__ bool add(float& acc, float2 v, Pixel p) const {
+    const float d1 = p.g - sqrtf(v.x * v.x + v.y * v.y);
+    const float x = 1.f + (d1 * d1) * p.inv;
+    float r = rsqrtf(x);
+    if (x < 1e30f) r = r * fmaf(-0.5f * x * r, r, 1.5f);
+    acc += r;
+    return true;
+  }
+  __device__ void add_odd(float&, float2, Pixel) const {}
+};
+
+// Row and column kernels of embedded frames; *run and *group_cols say where
+// the sums lie (for_each_sum).  The column kernel's runs fill the chip once.
+template <int N, class Op>
+cudaError_t embed_sum_t(const EmbedArgs& a, const Op& op, int* run, int* group_cols, int n_sms,
+                        cudaStream_t st) {
+  using ER = EmbedRows<N>;
+  constexpr int E = ER::E, LC = embed_group_cols(N);
+  const int sr = ER::kTotal * (int)sizeof(float2);
+  const int sc = (LC * padk(N, ER::SH) + tw_stage_total(N, E)) * (int)sizeof(float2);
+  cudaError_t e = cudaFuncSetAttribute(embed_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(embed_cols_sum_kernel<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
+  if (e != cudaSuccess) return e;
+  const int64_t total = (int64_t)(N / LC) * a.n, slots = (int64_t)embed_ctas(N) * n_sms;
+  *run = (int)((total + slots - 1) / slots);
+  *group_cols = LC;
+  const int64_t items = (int64_t)a.n * ((a.rows + ER::L - 1) / ER::L);
+  const int grid = (int)(items < n_sms * 3 ? items : n_sms * 3);
+  embed_rows_kernel<N><<<grid, kThreads, sr, st>>>(a);
+  embed_cols_sum_kernel<N, Op><<<(int)((total + *run - 1) / *run), kEmbedThreads, sc, st>>>(a, op, *run);
+  return cudaGetLastError();
+}
+
 template <int N>
 cudaError_t fft2_t(const float2* in, float2* out, int batch, int inverse, cudaStream_t st,
                    const float2* tw, int n_sms) {
@@ -109,9 +364,49 @@ cudaError_t fft2_t(const float2* in, float2* out, int batch, int inverse, cudaSt
 cudaError_t fft2_dispatch(const float2* in, float2* out, int N, int batch, int inverse,
                           cudaStream_t st);
 
+// embed_sum_t of F/|F| (goal null) or of the RFTF's summand (`work`: n N x N
+// planes)
+cudaError_t frame_sums_dispatch(int N, const float2* src, float2* work, int n, int rows, int cols,
+                                const float* goal, int* run, int* group_cols, cudaStream_t st);
+
+// The column kernel's partial sums (SumsAt: where they lie), added up and
+// transposed back: element (r, c) lies at row c, column r of their planes.  One
+// 32 x 32 tile per block (32 x 8 threads, grid of frame_sums_grid) through
+// shared memory; `f` gets each sum and its place.  N < 32: partial tiles.
+struct SumsAt {
+  int frames, run, group_cols;
+};
+inline dim3 frame_sums_grid(int N) { return dim3((N + 31) / 32, (N + 31) / 32); }
+template <class F>
+__device__ __forceinline__ void transposed_sums(const float2* __restrict__ part, SumsAt at, int N, F&& f) {
+  __shared__ float2 tile[32][33];
+  const int64_t NN = (int64_t)N * N;
+  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  for (int y = threadIdx.y; y < 32; y += 8) {
+    const int c = c0 + y, r = r0 + threadIdx.x;
+    if (c < N && r < N) {
+      float2 s = make_float2(0.f, 0.f);
+      for_each_sum(c, at.group_cols, at.frames, at.run, [&](int k) {
+        const float2 v = part[k * NN + (int64_t)c * N + r];
+        s.x += v.x;
+        s.y += v.y;
+      });
+      tile[y][threadIdx.x] = s;
+    }
+  }
+  __syncthreads();
+  for (int y = threadIdx.y; y < 32; y += 8) {
+    const int r = r0 + y, c = c0 + threadIdx.x;
+    if (c < N && r < N) f(r, c, tile[threadIdx.x][y]);
+  }
+}
+
 #define SP_DECLARE_FFT2(N) \
   cudaError_t fft2_n##N(const float2* in, float2* out, int batch, int inverse, cudaStream_t st, \
-                        const float2* tw, int n_sms);
+                        const float2* tw, int n_sms); \
+  cudaError_t phasor_frames_n##N(const EmbedArgs& a, int* run, int* group_cols, int n_sms, cudaStream_t st); \
+  cudaError_t rftf_frames_n##N(const EmbedArgs& a, const float* goal, int* run, int* group_cols, \
+                               int n_sms, cudaStream_t st);
 SP_DECLARE_FFT2(8)
 SP_DECLARE_FFT2(16)
 SP_DECLARE_FFT2(32)
@@ -127,6 +422,13 @@ SP_DECLARE_FFT2(4096)
   cudaError_t fft2_n##N(const float2* in, float2* out, int batch, int inverse, cudaStream_t st, \
                         const float2* tw, int n_sms) {                                        \
     return fft2_t<N>(in, out, batch, inverse, st, tw, n_sms);                                 \
+  }                                                                                           \
+  cudaError_t phasor_frames_n##N(const EmbedArgs& a, int* run, int* group_cols, int n_sms, cudaStream_t st) { \
+    return embed_sum_t<N>(a, PhasorSum{}, run, group_cols, n_sms, st);                        \
+  }                                                                                           \
+  cudaError_t rftf_frames_n##N(const EmbedArgs& a, const float* goal, int* run,               \
+                               int* group_cols, int n_sms, cudaStream_t st) {                 \
+    return embed_sum_t<N>(a, RftfSum{goal}, run, group_cols, n_sms, st);                      \
   }
 
 }  // namespace sp

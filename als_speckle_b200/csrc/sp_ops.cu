@@ -51,6 +51,25 @@ cudaError_t fft2_dispatch(const float2* in, float2* out, int N, int batch, int i
   }
 }
 
+cudaError_t frame_sums_dispatch(int N, const float2* src, float2* work, int n, int rows, int cols,
+                                const float* goal, int* run, int* group_cols, cudaStream_t st) {
+  const float2* tw = nullptr;
+  cudaError_t e = twiddles(&tw);
+  if (e != cudaSuccess) return e;
+  const int sms = n_sms_cached();
+  const EmbedArgs a{src, work, n, rows, cols, tw};
+  switch (N) {
+#define SP_CASE(N)                                                                   \
+  case N:                                                                            \
+    return goal ? rftf_frames_n##N(a, goal, run, group_cols, sms, st)                \
+                : phasor_frames_n##N(a, run, group_cols, sms, st);
+    SP_CASE(8) SP_CASE(16) SP_CASE(32) SP_CASE(64) SP_CASE(128)
+    SP_CASE(256) SP_CASE(512) SP_CASE(1024) SP_CASE(2048) SP_CASE(4096)
+#undef SP_CASE
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // elementwise operators (kernels/phasing_*.cl, common_abs_f2_f2.cl)
 // ---------------------------------------------------------------------------
@@ -141,7 +160,7 @@ __global__ void copy_to_buffer_kernel(float2* dst, const float2* src, int c0, in
 }
 // phasing_prtf_accumulate2.cl:16-25: |sum_n F_n/|F_n|| / frames
 __global__ void prtf_accumulate_kernel(int frames, const float2* __restrict__ fft,
-                                       float* __restrict__ prtf, int N, int shift) {
+                                       float* __restrict__ prtf, int N) {
   const int64_t NN = (int64_t)N * N;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < NN;
        k += (int64_t)gridDim.x * blockDim.x) {
@@ -156,32 +175,24 @@ __global__ void prtf_accumulate_kernel(int frames, const float2* __restrict__ ff
     }
     cr /= frames;
     ci /= frames;
-    int64_t dst = k;
-    if (shift) {  // np.fft.fftshift for even N
-      const int r = (int)(k / N), c = (int)(k - (int64_t)r * N);
-      dst = (int64_t)((r + N / 2) % N) * N + (c + N / 2) % N;
-    }
-    prtf[dst] = hypotf(cr, ci);
+    prtf[k] = hypotf(cr, ci);
   }
 }
 
-// sum_n F_n/|F_n| in FP32 (phasing_prtf_accumulate2.cl:20-23), added to acc
-__global__ void phasor_sum_kernel(int frames, const float2* __restrict__ fft, float2* __restrict__ acc,
-                                  int N) {
-  const int64_t NN = (int64_t)N * N;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < NN;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    float cr = 0.f, ci = 0.f;
-    for (int n = 0; n < frames; ++n) {
-      const float2 v = fft[k + n * NN];
-      const float h = hypotf(v.x, v.y);
-      if (h > 0.f) {
-        cr += v.x / h;
-        ci += v.y / h;
-      }
-    }
-    acc[k] = make_float2(acc[k].x + cr, acc[k].y + ci);
-  }
+// acc += the phasor sums
+__global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restrict__ part, SumsAt at,
+                                                         float2* __restrict__ acc, int N) {
+  transposed_sums(part, at, N, [&](int r, int c, float2 s) {
+    float2* p = acc + (int64_t)r * N + c;
+    *p = make_float2(p->x + s.x, p->y + s.y);
+  });
+}
+// prtf = fftshift(|phasor sums| / frames)
+__global__ void __launch_bounds__(256) prtf_sums_kernel(const float2* __restrict__ part, SumsAt at,
+                                                        float* __restrict__ prtf, int N) {
+  transposed_sums(part, at, N, [&](int r, int c, float2 s) {
+    prtf[(int64_t)((r + N / 2) % N) * N + (c + N / 2) % N] = hypotf(s.x / at.frames, s.y / at.frames);
+  });
 }
 // prtf = fftshift(|acc| / frames)
 __global__ void prtf_finish_kernel(const float2* __restrict__ acc, int frames, float* __restrict__ prtf,
@@ -192,19 +203,6 @@ __global__ void prtf_finish_kernel(const float2* __restrict__ acc, int frames, f
     const int r = (int)(k / N), c = (int)(k - (int64_t)r * N);
     const float2 a = acc[k];
     prtf[(int64_t)((r + N / 2) % N) * N + (c + N / 2) % N] = hypotf(a.x / frames, a.y / frames);
-  }
-}
-
-// embed (n, rows, cols) frames at the corner of zeroed N x N planes
-__global__ void embed_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int n,
-                             int rows, int cols, int N) {
-  const int64_t total = (int64_t)n * N * N;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t f = k / ((int64_t)N * N);
-    const int64_t rem = k - f * N * N;
-    const int r = (int)(rem / N), c = (int)(rem - (int64_t)r * N);
-    dst[k] = (r < rows && c < cols) ? src[(f * rows + r) * cols + c] : make_float2(0.f, 0.f);
   }
 }
 
@@ -546,7 +544,7 @@ int sp_copy_to_buffer_f2(void* dst, const void* src, int c0, int r0, int frame, 
 int sp_prtf_accumulate(int frames, const void* fft, float* prtf, int N, sp_stream_t stream) {
   SP_CHECK(fft && prtf && frames > 0 && N > 0, SP_ERR_INVALID, "sp_prtf_accumulate: bad argument");
   prtf_accumulate_kernel<<<grid_for((int64_t)N * N), 256, 0, as_stream(stream)>>>(
-      frames, (const float2*)fft, prtf, N, 0);
+      frames, (const float2*)fft, prtf, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }
@@ -584,13 +582,11 @@ int sp_prtf(const void* frames, int n_frames, int rows, int cols, int N, void* w
   SP_CHECK(rows > 0 && cols > 0 && rows <= N && cols <= N, SP_ERR_INVALID,
            "sp_prtf: frames larger than N");
   cudaStream_t st = as_stream(stream);
-  const int64_t total = (int64_t)n_frames * N * N;
-  embed_kernel<<<grid_for(total), 256, 0, st>>>((const float2*)frames, (float2*)work, n_frames, rows,
-                                                cols, N);
-  SP_CUDA_TRY(cudaGetLastError());
-  SP_CUDA_TRY(fft2_dispatch((const float2*)work, (float2*)work, N, n_frames, 0, st));
-  prtf_accumulate_kernel<<<grid_for((int64_t)N * N), 256, 0, st>>>(n_frames, (const float2*)work,
-                                                                   prtf, N, 1);
+  SumsAt at{n_frames, 1, 1};
+  SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, nullptr,
+                                  &at.run, &at.group_cols, st));
+  prtf_sums_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>(
+      (const float2*)work, at, prtf, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }
@@ -602,13 +598,11 @@ int sp_prtf_phasors(const void* frames, int n_frames, int rows, int cols, int N,
   SP_CHECK(rows > 0 && cols > 0 && rows <= N && cols <= N, SP_ERR_INVALID,
            "sp_prtf_phasors: frames larger than N");
   cudaStream_t st = as_stream(stream);
-  const int64_t total = (int64_t)n_frames * N * N;
-  embed_kernel<<<grid_for(total), 256, 0, st>>>((const float2*)frames, (float2*)work, n_frames, rows,
-                                                cols, N);
-  SP_CUDA_TRY(cudaGetLastError());
-  SP_CUDA_TRY(fft2_dispatch((const float2*)work, (float2*)work, N, n_frames, 0, st));
-  phasor_sum_kernel<<<grid_for((int64_t)N * N), 256, 0, st>>>(n_frames, (const float2*)work,
-                                                              (float2*)acc, N);
+  SumsAt at{n_frames, 1, 1};
+  SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, nullptr,
+                                  &at.run, &at.group_cols, st));
+  phasor_sum_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>(
+      (const float2*)work, at, (float2*)acc, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }

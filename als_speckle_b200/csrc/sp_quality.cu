@@ -97,6 +97,14 @@ __global__ void rftf_accumulate_kernel(int frames, const float* goal, float* acc
   }
 }
 
+// acc = fftshift(the RFTF sums / frames)
+__global__ void __launch_bounds__(256) rftf_sums_kernel(const float2* __restrict__ part, SumsAt at,
+                                                        float* __restrict__ acc, int N) {
+  transposed_sums(part, at, N, [&](int r, int c, float2 s) {
+    acc[(int64_t)((r + N / 2) % N) * N + (c + N / 2) % N] = s.x / (float)at.frames;
+  });
+}
+
 // FP64 sums[0] = sum |F - g|, sums[1] = sum |shift(F) - g| (rftf's choice
 // between a goal modulus centred at (0,0) and at (N/2,N/2), phasing.py:1583-1584);
 // F is the real part of `fourier`.
@@ -277,6 +285,22 @@ int sp_rftf_accumulate(int frames, const float* goal, float* accumulation, const
            "sp_rftf_accumulate: bad argument");
   rftf_accumulate_kernel<<<grid_of((int64_t)N * N), 256, 0, as_stream(stream)>>>(
       frames, goal, accumulation, (const float2*)fourier, N, shift);
+  SP_CUDA_TRY(cudaGetLastError());
+  return SP_OK;
+}
+
+int sp_rftf_frames(const void* frames, int n_frames, int rows, int cols, const float* goal, int N,
+                   void* work, float* accumulation, sp_stream_t stream) {
+  SP_N_CHECK(N, "sp_rftf_frames");
+  SP_CHECK(frames && goal && work && accumulation && n_frames > 0, SP_ERR_INVALID,
+           "sp_rftf_frames: bad argument");
+  SP_CHECK(rows > 0 && cols > 0 && rows <= N && cols <= N, SP_ERR_INVALID,
+           "sp_rftf_frames: frames larger than N");
+  cudaStream_t st = as_stream(stream);
+  SumsAt at{n_frames, 1, 1};
+  SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, goal,
+                                  &at.run, &at.group_cols, st));
+  rftf_sums_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>((const float2*)work, at, accumulation, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }

@@ -872,11 +872,17 @@ def gpu_rftf(gpuinfo, estimates, goal_modulus, ipsf=None, rftfq=False):
         if isinstance(goal_modulus, np.ndarray) else goal_modulus.to(torch.float32).contiguous()
     N = int(g.shape[0])
     _pow2_size(N, "gpu_rftf")
-    L = est.shape[0]
+    L, rows, cols = est.shape
     st = stream_ptr()
-    f = _embed(est, N)
-    call("sp_fft2", ptr(f), ptr(f), N, L, 0, st)
-    if ipsf is not None:
+    acc = torch.empty((N, N), dtype=torch.float32, device=g.device)
+    if ipsf is None:
+        if rows > N or cols > N:
+            raise ValueError("estimate must be smaller than goal_modulus")
+        work = torch.empty((L, N, N), dtype=torch.complex64, device=est.device)
+        call("sp_rftf_frames", ptr(est), L, rows, cols, ptr(g), N, ptr(work), ptr(acc), st)
+    else:
+        f = _embed(est, N)
+        call("sp_fft2", ptr(f), ptr(f), N, L, 0, st)
         ip = np.real(np.asarray(ipsf)).astype(np.float32) if not isinstance(ipsf, torch.Tensor) \
             else ipsf.real.cpu().numpy().astype(np.float32)
         ipd = torch.from_numpy(np.ascontiguousarray(ip)).cuda()
@@ -885,10 +891,7 @@ def gpu_rftf(gpuinfo, estimates, goal_modulus, ipsf=None, rftfq=False):
         call("sp_multiply_axis_f_f2", L, ptr(ipd), ptr(f), ptr(f), N * N, st)
         call("sp_fft2", ptr(f), ptr(f), N, L, 1, st)
         call("sp_sqrt_f2", ptr(f), ptr(f), f.numel(), st)
-    else:
-        call("sp_abs_f2_f2", ptr(f), ptr(f), f.numel(), st)
-    acc = torch.empty((N, N), dtype=torch.float32, device=g.device)
-    call("sp_rftf_accumulate", L, ptr(g), ptr(acc), ptr(f), N, 1, st)
+        call("sp_rftf_accumulate", L, ptr(g), ptr(acc), ptr(f), N, 1, st)
     res = acc.cpu().numpy() if was_np else acc
     if rftfq:
         return res, unwrap_average(acc, as_numpy=was_np)

@@ -280,6 +280,10 @@ int sp_multiply_f2_f2(const void* a_dev, const void* b_dev, void* out_dev, int64
  * acc = mean over frames of 1/sqrt(1 + (g - Re F)^2/g^2), written fftshifted if shift. */
 int sp_rftf_accumulate(int frames, const float* goal_dev, float* accumulation_dev,
                        const void* fourier_dev, int N, int shift, sp_stream_t stream);
+/* the same from the estimates themselves, fftshifted: frames (n_frames, rows, cols) embedded
+ * at the corner of N x N, F = |FFT2|.  work_dev: complex64 n_frames*N*N scratch. */
+int sp_rftf_frames(const void* frames_dev, int n_frames, int rows, int cols, const float* goal_dev,
+                   int N, void* work_dev, float* accumulation_dev, sp_stream_t stream);
 /* rftf's error map for one estimate (phasing.py:1583-1601): picks the goal's centring from
  * the FP64 sums |F - g| and |shift(F) - g| (sums_dev: 2 doubles, read back), writes the
  * centred error err_dev and out_dev = sqrt(1/(1+err)) (rescaled to [0,1] if scale). */

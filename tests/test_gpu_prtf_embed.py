@@ -1,0 +1,62 @@
+"""PRTF phasor sums of embedded frames (rows and columns fewer than N, chunks
+of frames) at every transform size, against FP64 numpy.
+
+Bound: a phasor's error is the transform's error over |F|.  The transform of
+white noise is good to ~3e-7 of its rms (the FFT's own bound here is 2e-6
+relative norm); |F|^2 is exponentially distributed, so the least of P pixels
+times F frames is ~rms/sqrt(P F) >= rms/1500 at these sizes, and one frame's
+phasor weighs 1/F: 2e-6 * 1500 / F per pixel at worst."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,frames,rows,cols", [
+    (8, 3, 8, 8), (8, 5, 3, 7), (16, 4, 9, 16), (32, 7, 32, 5), (64, 33, 17, 40), (128, 20, 101, 67),
+    (256, 9, 180, 181), (512, 5, 512, 1), (512, 13, 173, 400), (1024, 2, 33, 1000), (2048, 2, 70, 51),
+    (4096, 1, 33, 65)])
+def test_prtf_of_embedded_frames(N, frames, rows, cols):
+    import torch
+    from als_speckle_b200.phasing import prtf
+    from als_speckle_b200._lib import call, ptr, stream_ptr
+    rng = np.random.default_rng(N + frames)
+    x = (rng.standard_normal((frames, rows, cols)) + 1j * rng.standard_normal((frames, rows, cols)))
+    x = x.astype(np.complex64)
+    acc = np.zeros((N, N), np.complex128)
+    for f in x:
+        F = np.fft.fft2(f.astype(np.complex128), s=(N, N))
+        acc += F / np.abs(F)
+    t = torch.from_numpy(x).cuda()
+    tol = 2e-6 * 1500 / frames
+    got = prtf(t, N=N).cpu().numpy()
+    assert np.max(np.abs(got - np.fft.fftshift(np.abs(acc) / frames))) < tol
+    # the two halves: phasor sums added to what acc holds, in its own layout
+    out = torch.full((N, N), 1.5 - 0.5j, dtype=torch.complex64, device="cuda")
+    work = torch.empty((frames, N, N), dtype=torch.complex64, device="cuda")
+    call("sp_prtf_phasors", ptr(t), frames, rows, cols, N, ptr(work), ptr(out), stream_ptr())
+    assert np.max(np.abs(out.cpu().numpy() - (acc + 1.5 - 0.5j))) < tol * frames
+
+
+@pytest.mark.parametrize("N,frames,rows,cols", [
+    (8, 3, 8, 8), (16, 4, 9, 16), (64, 33, 17, 40), (256, 9, 180, 181), (512, 13, 173, 400),
+    (1024, 2, 33, 1000), (4096, 1, 33, 65)])
+def test_rftf_of_embedded_frames(N, frames, rows, cols):
+    """gpu_rftf without an ipsf against FP64 numpy.  A summand's slope in |F|
+    is at most 0.385/g; with g >= 0.2 rms and a pixel's transform good to 1e-5
+    of the rms (2e-6 in norm) it is good to 2e-5.  Where g = 0 it is 0."""
+    import torch
+    from als_speckle_b200.phasing import gpu_rftf
+    rng = np.random.default_rng(N + frames)
+    x = (rng.standard_normal((frames, rows, cols)) + 1j * rng.standard_normal((frames, rows, cols)))
+    x = x.astype(np.complex64)
+    rms = np.sqrt(2.0 * rows * cols)
+    g = ((0.2 + 2 * rng.random((N, N))) * rms).astype(np.float32)
+    g[N // 3, N // 5] = 0
+    want = np.zeros((N, N))
+    with np.errstate(divide="ignore"):
+        for f in x:
+            F = np.abs(np.fft.fft2(f.astype(np.complex128), s=(N, N)))
+            want += 1 / np.sqrt(1 + (g.astype(np.float64) - F) ** 2 / g.astype(np.float64) ** 2)
+    got = gpu_rftf(None, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()).cpu().numpy()
+    assert np.max(np.abs(got - np.fft.fftshift(want / frames))) < 2e-5
