@@ -1,10 +1,12 @@
-// Engine kernels, standalone 2-D FFT and partial-coherence kernels for N = 128 (see
-// sp_engine_launch.cuh, sp_fft2.cuh and sp_coherence.cuh).
+// Engine kernels, standalone 2-D FFT, partial-coherence and registration kernels for
+// N = 128 (see sp_engine_launch.cuh, sp_fft2.cuh, sp_coherence.cuh and sp_register.cuh).
 #include "sp_engine_launch.cuh"
 #include "sp_fft2.cuh"
 #include "sp_coherence.cuh"
+#include "sp_register.cuh"
 namespace sp {
 SP_DEFINE_SIZE(128)
 SP_DEFINE_FFT2(128)
 SP_DEFINE_PC(128)
+SP_DEFINE_REG(128)
 }  // namespace sp

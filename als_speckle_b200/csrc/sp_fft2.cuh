@@ -101,27 +101,34 @@ struct EmbedArgs {
   const float2* tw;
 };
 
-constexpr int kEmbedThreads = 128;  // column kernel
+constexpr int kEmbedThreads = 128;  // CTAs of the column kernel
 // values per thread: those of sp_fft2, so that the transforms are its bit for
 // bit (where F is nearly 0 its phasor amplifies any change of rounding), but
-// for 4096 points, which need 128 threads
+// for columns of 4096 points, which would need 256 threads
 __host__ __device__ constexpr int embed_e(int N) { return N >= 4096 ? 32 : (N < 16 ? N : 16); }
-// resident CTAs per SM the kernels are compiled for
+// resident CTAs per SM it is compiled for
 __host__ __device__ constexpr int embed_ctas(int N) { return embed_e(N) > 16 ? 3 : 5; }
 
-// The row kernel's lines, in strips whose pitch (as the column pass's) makes
-// the transposed reads, L rows of 16 / L columns per half-warp, conflict-free.
+// ---------------------------------------------------------------------------
+// Lines of planes transformed one by one: a CTA takes L lines of one plane, T
+// threads each, with no barrier wider than the line around the transform.  The
+// Op supplies line values and takes the results; transposed_store writes them
+// out with line and position exchanged, so that the other dimension's lines
+// are contiguous for the next kernel.  The strips' pitch (as the column
+// pass's) makes its reads, L lines of 16 / L positions per half-warp,
+// conflict-free.  E = min(16, N) as in sp_fft2: bitwise its transforms.
+// ---------------------------------------------------------------------------
 template <int N>
-struct EmbedRows {
-  static constexpr int E = embed_e(N), T = N / E, L = lines_per_item(N, E), SH = pad_shift(E);
+struct Lines {
+  static constexpr int E = (N < 16 ? N : 16), T = N / E, L = lines_per_item(N, E), SH = pad_shift(E);
   static constexpr int P = L >= 16 ? next_congruent(padk(N, SH), 1, 2)
                                    : next_congruent(padk(N, SH), 16 / L, 16);
   static constexpr int kTw = L * P;
-  static constexpr int kTotal = kTw + tw_stage_total(N, E);
+  static constexpr int kExtra = kTw + tw_stage_total(N, E);  // the Op's own, Op::extra(N) entries
 };
 
 template <int T>
-struct EmbedSync {
+struct LineGroupSync {
   using type = typename std::conditional<(T <= 32), WarpSync, LineSync<T>>::type;
   __device__ static type make(int line) {
     if constexpr (T <= 32) return type{};
@@ -129,48 +136,99 @@ struct EmbedSync {
   }
 };
 
-template <int N>
-__global__ void __launch_bounds__(kThreads, embed_e(N) > 16 ? 1 : 3) embed_rows_kernel(EmbedArgs a) {
-  using ER = EmbedRows<N>;
-  constexpr int E = ER::E, T = ER::T, L = ER::L, SH = ER::SH;
+// dst[pos * pitch + l] = value of line l at `pos`, for l < nl and pos < np.
+// Every thread of the block calls it; the strips are free afterwards.
+template <int N, class Sync>
+__device__ __forceinline__ void transposed_store(const float2 (&v)[Lines<N>::E], float2* smem, int lrow,
+                                                 int t, const Sync& sync, float2* dst, size_t pitch,
+                                                 int nl, int np) {
+  using LN = Lines<N>;
+  const RowLayout<LN::SH> lay{smem + (lrow < LN::L ? lrow : 0) * LN::P};
+  sync();  // the line's last stage has read its strip
+  if (lrow < LN::L) {
+#pragma unroll
+    for (int i = 0; i < LN::E; ++i) lay.at(t + i * LN::T) = v[i];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < LN::L * np; q += kThreads) {
+    const int l = q % LN::L, pos = q / LN::L;
+    if (l < nl) dst[(size_t)pos * pitch + l] = smem[l * LN::P + padk(pos, LN::SH)];
+  }
+  __syncthreads();
+}
+
+// Op: planes, lines (of a plane), extra(N) (float2 entries of shared memory of
+// its own), init(extra) (once per CTA) and prepare(plane, extra) (at each new
+// plane; block-wide, it synchronises if it writes), line(plane, line) -> Line, what the
+// line's threads keep of it, load(Line, pos, extra), done(plane, line0, nl, v,
+// smem, lrow, t, sync).
+template <int N, int DIR, class Op>
+__global__ void __launch_bounds__(kThreads, 3) lines_kernel(Op op, const float2* __restrict__ tw_all) {
+  using LN = Lines<N>;
+  constexpr int E = LN::E, T = LN::T, L = LN::L;
   extern __shared__ float2 smem[];
-  float2* tw = smem + ER::kTw;
-  build_stage_twiddles<N, E>(tw, a.tw + N);
+  float2* tw = smem + LN::kTw;
+  float2* extra = smem + LN::kExtra;
+  build_stage_twiddles<N, E>(tw, tw_all + N);
+  op.init(extra);
   __syncthreads();
   const int lrow = threadIdx.x / T;
   const int t = threadIdx.x - lrow * T;
   const bool line = lrow < L;
-  const RowLayout<SH> lay{smem + (line ? lrow : 0) * ER::P};
-  const auto sync = EmbedSync<T>::make(lrow);
-  const int blocks = (a.rows + L - 1) / L;  // of one frame
-  const int64_t items = (int64_t)a.n * blocks;
-  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-    const int64_t f = it / blocks;
-    const int r0 = (int)(it - f * blocks) * L;
-    const bool mine = line && r0 + lrow < a.rows;
-    const float2* src = a.src + (f * a.rows + r0 + (mine ? lrow : 0)) * a.cols;
+  const RowLayout<LN::SH> lay{smem + (line ? lrow : 0) * LN::P};
+  const auto sync = LineGroupSync<T>::make(lrow);
+  const int blocks = (op.lines + L - 1) / L;  // of one plane
+  const int64_t items = (int64_t)op.planes * blocks;
+  // each CTA a run of neighbouring items, so that it prepares few planes
+  const int64_t run = (items + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * run;
+  int ready = -1;
+  for (int64_t it = i0; it < items && it < i0 + run; ++it) {
+    const int f = (int)(it / blocks);
+    const int l0 = (int)(it - (int64_t)f * blocks) * L;
+    const int nl = op.lines - l0 < L ? op.lines - l0 : L;
+    if (f != ready) op.prepare(f, extra);
+    ready = f;
+    const typename Op::Line ln = op.line(f, l0 + (lrow < nl ? lrow : 0));
     float2 v[E];
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-      const int c = t + i * T;
-      v[i] = (mine && c < a.cols) ? src[c] : make_float2(0.f, 0.f);
-    }
-    fft_line<N, E, -1>(v, lay, sync, line, t, tw);
-    sync();  // the line's last stage has read its strip
-    if (line) {
-#pragma unroll
-      for (int i = 0; i < E; ++i) lay.at(t + i * T) = v[i];
-    }
-    __syncthreads();
-    const int nr = a.rows - r0 < L ? a.rows - r0 : L;
-    float2* dst = a.dst + f * N * N + r0;
-    for (int q = threadIdx.x; q < L * N; q += kThreads) {
-      const int r = q % L, c = q / L;
-      if (r < nr) dst[(size_t)c * N + r] = smem[r * ER::P + padk(c, SH)];
-    }
-    __syncthreads();  // the strips are free
+    for (int i = 0; i < E; ++i)
+      v[i] = lrow < nl ? op.load(ln, t + i * T, extra) : make_float2(0.f, 0.f);
+    fft_line<N, E, DIR>(v, lay, sync, line, t, tw);
+    op.template done<N>(f, l0, nl, v, smem, lrow, t, sync);
   }
 }
+
+template <int N, int DIR, class Op>
+cudaError_t launch_lines(const Op& op, const float2* tw, int n_sms, cudaStream_t st) {
+  const int sm = (Lines<N>::kExtra + Op::extra(N)) * (int)sizeof(float2);
+  const cudaError_t e =
+      cudaFuncSetAttribute(lines_kernel<N, DIR, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  if (e != cudaSuccess) return e;
+  const int64_t items = (int64_t)op.planes * ((op.lines + Lines<N>::L - 1) / Lines<N>::L);
+  if (items == 0) return cudaSuccess;
+  lines_kernel<N, DIR, Op><<<(int)(items < n_sms * 3 ? items : n_sms * 3), kThreads, sm, st>>>(op, tw);
+  return cudaGetLastError();
+}
+
+// The frames' rows, zero-padded to N, stored transposed into the planes.
+struct EmbedRowsOp {
+  const float2* src;
+  float2* dst;
+  int planes, lines, cols;  // lines: rows of a frame
+  static constexpr int extra(int) { return 0; }
+  __device__ void init(float2*) const {}
+  __device__ void prepare(int, float2*) const {}
+  using Line = const float2*;
+  __device__ __forceinline__ Line line(int f, int r) const { return src + ((int64_t)f * lines + r) * cols; }
+  __device__ __forceinline__ float2 load(Line l, int c, const float2*) const {
+    return c < cols ? l[c] : make_float2(0.f, 0.f);
+  }
+  template <int N, class Sync>
+  __device__ __forceinline__ void done(int f, int l0, int nl, const float2 (&v)[Lines<N>::E],
+                                       float2* smem, int lrow, int t, const Sync& sync) const {
+    transposed_store<N>(v, smem, lrow, t, sync, dst + (size_t)f * N * N + l0, N, nl, N);
+  }
+};
 
 // Columns of the transposed planes, one line of T threads each.  The work is
 // the (column group, frame) pairs, groups outermost, dealt to the CTAs in equal
@@ -195,7 +253,7 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
   const int t = threadIdx.x - lc * T;
   const bool active = lc < L;
   const RowLayout<SH> lay{smem + (active ? lc : 0) * padk(N, SH)};
-  const auto sync = EmbedSync<T>::make(lc);
+  const auto sync = LineGroupSync<T>::make(lc);
   const int64_t total = (int64_t)(N / L) * a.n;
   int64_t u = (int64_t)blockIdx.x * run;
   const int64_t end = u + run < total ? u + run : total;
@@ -316,20 +374,15 @@ struct RftfSum {
 template <int N, class Op>
 cudaError_t embed_sum_t(const EmbedArgs& a, const Op& op, int* run, int* group_cols, int n_sms,
                         cudaStream_t st) {
-  using ER = EmbedRows<N>;
-  constexpr int E = ER::E, LC = embed_group_cols(N);
-  const int sr = ER::kTotal * (int)sizeof(float2);
-  const int sc = (LC * padk(N, ER::SH) + tw_stage_total(N, E)) * (int)sizeof(float2);
-  cudaError_t e = cudaFuncSetAttribute(embed_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sr);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(embed_cols_sum_kernel<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
+  constexpr int E = embed_e(N), LC = embed_group_cols(N);
+  const int sc = (LC * padk(N, pad_shift(E)) + tw_stage_total(N, E)) * (int)sizeof(float2);
+  cudaError_t e = cudaFuncSetAttribute(embed_cols_sum_kernel<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
   if (e != cudaSuccess) return e;
   const int64_t total = (int64_t)(N / LC) * a.n, slots = (int64_t)embed_ctas(N) * n_sms;
   *run = (int)((total + slots - 1) / slots);
   *group_cols = LC;
-  const int64_t items = (int64_t)a.n * ((a.rows + ER::L - 1) / ER::L);
-  const int grid = (int)(items < n_sms * 3 ? items : n_sms * 3);
-  embed_rows_kernel<N><<<grid, kThreads, sr, st>>>(a);
+  e = launch_lines<N, -1>(EmbedRowsOp{a.src, a.dst, a.n, a.rows, a.cols}, a.tw, n_sms, st);
+  if (e != cudaSuccess) return e;
   embed_cols_sum_kernel<N, Op><<<(int)((total + *run - 1) / *run), kEmbedThreads, sc, st>>>(a, op, *run);
   return cudaGetLastError();
 }

@@ -23,16 +23,11 @@
 #include <algorithm>
 #include <cmath>
 
-#include "sp_common.cuh"
+#include "sp_register.cuh"
 
 namespace sp {
 
-cudaError_t fft2_dispatch(const float2* in, float2* out, int N, int batch, int inverse,
-                          cudaStream_t st);
-
 static inline int upsampled_points(int U) { return (3 * U + 1) / 2; }  // ceil(1.5 U)
-
-__device__ __forceinline__ int signed_freq(int k, int N) { return k >= N / 2 ? k - N : k; }
 
 // exp(2 pi i num / den) with num reduced modulo den exactly first
 __device__ __forceinline__ float2 turn(long long num, long long den) {
@@ -42,67 +37,6 @@ __device__ __forceinline__ float2 turn(long long num, long long den) {
   sincospif(2.0f * (float)((double)r / (double)den), &s, &c);
   return make_float2(c, s);
 }
-// the same for a power-of-two denominator N: the residue is a mask (two's
-// complement gives the non-negative residue of a negative numerator too)
-__device__ __forceinline__ float2 turn_pow2(int num, int N) {
-  float s, c;
-  sincospif(2.0f * (float)(num & (N - 1)) / (float)N, &s, &c);
-  return make_float2(c, s);
-}
-
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
-  return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
-
-// frames (n, rows, cols) at the corner of zeroed N x N planes
-__global__ void reg_embed_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int n,
-                                 int rows, int cols, int N) {
-  const long long total = (long long)n * N * N;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x) {
-    const long long f = k / ((long long)N * N);
-    const long long rem = k - f * N * N;
-    const int r = (int)(rem / N), c = (int)(rem - (long long)r * N);
-    dst[k] = (r < rows && c < cols) ? src[(f * rows + r) * cols + c] : make_float2(0.f, 0.f);
-  }
-}
-
-// X_f = F_f conj(R)
-__global__ void reg_cross_kernel(const float2* __restrict__ F, const float2* __restrict__ R,
-                                 float2* __restrict__ X, int n, long long NN) {
-  const long long total = (long long)n * NN;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x)
-    X[k] = cmulc(F[k], R[k % NN]);
-}
-
-// per frame: max over the fftshifted |c_f|, keyed (|c| bits << 32 | ~index)
-__global__ void reg_argmax_kernel(const float2* __restrict__ C, int N,
-                                  unsigned long long* __restrict__ best) {
-  const int f = blockIdx.y;
-  const long long NN = (long long)N * N;
-  const float2* c = C + f * NN;
-  unsigned long long mine = 0;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < NN;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(k / N), cc = (int)(k - (long long)r * N);
-    const uint32_t sidx = (uint32_t)(((r + N / 2) % N) * N + (cc + N / 2) % N);
-    const float2 v = c[k];
-    const float m = sqrtf(v.x * v.x + v.y * v.y);
-    const unsigned long long key = ((unsigned long long)__float_as_uint(m) << 32) | (0xffffffffu - sidx);
-    mine = key > mine ? key : mine;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long other = __shfl_xor_sync(0xffffffffu, mine, o);
-    mine = other > mine ? other : mine;
-  }
-  if ((threadIdx.x & 31) == 0) atomicMax(&best[f], mine);
-}
-
 // the signed coarse shift d0 of frame f from its argmax key
 __device__ __forceinline__ int2 coarse_shift(unsigned long long key, int N) {
   const uint32_t sidx = 0xffffffffu - (uint32_t)(key & 0xffffffffu);
@@ -118,122 +52,181 @@ __global__ void reg_kernel_table(float2* __restrict__ W, int N, int U, int M) {
   }
 }
 
-// T1[f][ky][q] = sum_kx X_f'[ky][kx] W[kx][q], X_f' = F_f conj(R) exp(2 pi i k.d0/N).
-// CTA: 32 rows ky of one frame, all M columns; kx in chunks of 32 through
-// shared memory.  The modulation is separable, exp(2 pi i ky d0y/N) times
-// exp(2 pi i kx d0x/N): the CTA's row factors are made once, each chunk's
-// column factors once per chunk.  Thread (tr, tq) accumulates the register
-// tile of rows tr + 8 j (j < 4) and columns tq + 32 m (m < 8, up to M).
-constexpr int kRegRows = 32, kRegK = 32, kRegThreads = 256;
-__global__ void __launch_bounds__(kRegThreads) reg_upsample_rows_kernel(
-    const float2* __restrict__ F, const float2* __restrict__ R, const float2* __restrict__ W,
-    const unsigned long long* __restrict__ best, float2* __restrict__ T1, int N, int M) {
-  extern __shared__ float2 sm[];
-  float2* xs = sm;                           // [kRegRows][kRegK + 1]
-  float2* ws = sm + kRegRows * (kRegK + 1);  // [kRegK][M]
-  __shared__ float2 rowf[kRegRows], colf[kRegK];
-  const int f = blockIdx.y;
-  const int ky0 = blockIdx.x * kRegRows;
-  const long long NN = (long long)N * N;
-  const int2 d0 = coarse_shift(best[f], N);
-  const float2* Ff = F + f * NN;
-  if (threadIdx.x < kRegRows) rowf[threadIdx.x] = turn_pow2(signed_freq(ky0 + threadIdx.x, N) * d0.x, N);
-  const int tr = threadIdx.x / 32, tq = threadIdx.x % 32;
-  constexpr int MQ = 8;  // up to 256 columns
-  float2 acc[4][MQ];
+// The upsampled DFT is two complex matrix products, C[i][q] = sum_k A[i][k]
+// B[k][q], added up over k in order in FP32 (the peak search compares values
+// that differ in the last digits, so the order is part of the result):
+//   rows: A = X_f' = F_f conj(R) exp(2 pi i k.d0/N)  (i = ky, k = kx), B = W,
+//         C = T1_f, stored
+//   cols: A = W^T (i = p, k = ky), B = T1_f; C = the correlation on the fine
+//         grid, only its largest |c| kept (ties to the first index p M + q)
+// Bound by the FMA pipes: four FMAs per term, as two packed FP32x2
+// instructions per term on the real or imaginary parts of two rows i,
+//   re += (-a.y b.y), then += a.x b.x;   im += a.y b.x, then += a.x b.y
+// (each lane in the order of the scalar form).  A CTA takes 4 R rows and all M
+// columns, a warp R rows, whose A values are broadcasts of (re, re, im, im) of
+// a row pair from shared memory, and a lane the columns lane + 32 m, m < MQ.
+// Shared memory is the next limit (pairing re with im instead needs twice the A
+// loads and ran at its bandwidth: 245 us), so a warp keeps R as large as the
+// registers allow; four 128-thread CTAs per SM cover one another's staging.
+// 128 frames, N = 256, M = 96: rows 178 us (FMA pipes 62% busy) and columns
+// 69 us; 557 and 234 us with scalar FMAs on 4 x 3 and 1 x 3 tiles.
+constexpr int kRegK = 32, kRegThreads = 128, kRegWarps = kRegThreads / 32;
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{.reg .b64 ra, rb, rc, rr;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.ftz.f32x2 rr, ra, rb, rc;\n\tmov.b64 {%0, %1}, rr;}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+// row pairs of a warp for MQ column groups: 48-64 accumulator registers
+__host__ __device__ constexpr int reg_pairs(int MQ) { return MQ <= 4 ? 4 : 2; }
+__host__ __device__ constexpr int reg_tile_rows(int MQ) { return kRegWarps * 2 * reg_pairs(MQ); }
+
+// re[j][m], im[j][m]: the two rows of the warp's pair j, column lane + 32 m.
+// `as` holds [pair of the tile][k], `bs` [k][M].
+template <int MQ, class Src>
+__device__ __forceinline__ void reg_product(float2 (&re)[reg_pairs(MQ)][MQ],
+                                            float2 (&im)[reg_pairs(MQ)][MQ], const Src& src, int K, int M,
+                                            float4* as, float2* bs) {
+  constexpr int R = reg_pairs(MQ);
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
+  for (int j = 0; j < R; ++j)
 #pragma unroll
-    for (int m = 0; m < MQ; ++m) acc[j][m] = make_float2(0.f, 0.f);
-  for (int kx0 = 0; kx0 < N; kx0 += kRegK) {
+    for (int m = 0; m < MQ; ++m) re[j][m] = im[j][m] = make_float2(0.f, 0.f);
+  for (int k0 = 0; k0 < K; k0 += kRegK) {
+    const int nk = K - k0 < kRegK ? K - k0 : kRegK;  // K = N: 8 and 16 are shorter
     __syncthreads();  // the previous chunk's tiles are consumed
-    if (threadIdx.x < kRegK) colf[threadIdx.x] = turn_pow2(signed_freq(kx0 + threadIdx.x, N) * d0.y, N);
+    // nk rows of B are contiguous; nk and k0 are multiples of 8, so they are
+    // whole 16-byte pieces
+    for (int i = threadIdx.x; i < nk * M / 2; i += kRegThreads)
+      cp_async<16>(bs + 2 * i, src.b + (size_t)k0 * M + 2 * i);
+    src.stage(k0, nk, as, kRegWarps * R);
+    cp_async_wait_all();
     __syncthreads();
-    for (int i = threadIdx.x; i < kRegRows * kRegK; i += blockDim.x) {
-      const int rr = i / kRegK, kk = i - rr * kRegK;
-      const int ky = ky0 + rr, kx = kx0 + kk;
-      float2 v = make_float2(0.f, 0.f);
-      if (ky < N && kx < N) {
-        const long long idx = (long long)ky * N + kx;
-        v = cmul(cmul(cmulc(Ff[idx], R[idx]), rowf[rr]), colf[kk]);
-      }
-      xs[rr * (kRegK + 1) + kk] = v;
-    }
-    for (int i = threadIdx.x; i < kRegK * M; i += blockDim.x) {
-      const int kk = i / M, q = i - kk * M;
-      ws[i] = (kx0 + kk < N) ? W[(long long)(kx0 + kk) * M + q] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    for (int kk = 0; kk < kRegK; ++kk) {
-      float2 x[4];
+#pragma unroll 4
+    for (int kk = 0; kk < nk; ++kk) {
+      float4 a[R];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) x[j] = xs[(tr + 8 * j) * (kRegK + 1) + kk];
+      for (int j = 0; j < R; ++j) a[j] = as[(w * R + j) * kRegK + kk];
 #pragma unroll
       for (int m = 0; m < MQ; ++m) {
-        const int q = tq + 32 * m;
-        if (q < M) {
-          const float2 w = ws[kk * M + q];
+        const int q = lane + 32 * m;
+        const float2 b = bs[kk * M + (q < M ? q : 0)];
+        const float2 bx = make_float2(b.x, b.x), by = make_float2(b.y, b.y);
+        const float2 ny = make_float2(-b.y, -b.y);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[j][m].x = fmaf(x[j].x, w.x, fmaf(-x[j].y, w.y, acc[j][m].x));
-            acc[j][m].y = fmaf(x[j].x, w.y, fmaf(x[j].y, w.x, acc[j][m].y));
-          }
+        for (int j = 0; j < R; ++j) {
+          const float2 ar = make_float2(a[j].x, a[j].y), ai = make_float2(a[j].z, a[j].w);
+          re[j][m] = fma2(ar, bx, fma2(ai, ny, re[j][m]));
+          im[j][m] = fma2(ar, by, fma2(ai, bx, im[j][m]));
         }
       }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int ky = ky0 + tr + 8 * j;
-    if (ky >= N) continue;
-#pragma unroll
-    for (int m = 0; m < MQ; ++m) {
-      const int q = tq + 32 * m;
-      if (q < M) T1[((long long)f * N + ky) * M + q] = acc[j][m];
     }
   }
 }
 
-// c_f[p][q] = sum_ky W[ky][p] T1_f[ky][q]; CTA: 8 rows p of one frame, all
-// M columns; the CTA's largest |c| goes into best_up[f] (ties to the first
-// index p M + q).
-__global__ void __launch_bounds__(kRegThreads) reg_upsample_cols_kernel(
-    const float2* __restrict__ T1, const float2* __restrict__ W, int N, int M,
-    unsigned long long* __restrict__ best_up) {
-  const int f = blockIdx.y;
-  const int p0 = blockIdx.x * 8;
-  const int tp = threadIdx.x / 32, tq = threadIdx.x % 32;
-  const int p = p0 + tp;
-  constexpr int MQ = 8;
-  float2 acc[MQ];
-#pragma unroll
-  for (int m = 0; m < MQ; ++m) acc[m] = make_float2(0.f, 0.f);
-  const float2* t1 = T1 + (long long)f * N * M;
-  if (p < M) {
-    for (int ky = 0; ky < N; ++ky) {
-      const float2 w = W[(long long)ky * M + p];
-#pragma unroll
-      for (int m = 0; m < MQ; ++m) {
-        const int q = tq + 32 * m;
-        if (q < M) {
-          const float2 t = t1[(long long)ky * M + q];
-          acc[m].x = fmaf(w.x, t.x, fmaf(-w.y, t.y, acc[m].x));
-          acc[m].y = fmaf(w.x, t.y, fmaf(w.y, t.x, acc[m].y));
-        }
+// A = X_f' of one frame's rows ky0 ..: the modulation is separable, the row
+// factors exp(2 pi i ky d0y/N) made once, a chunk's column factors once each.
+struct RegRowsSrc {
+  const float2 *F, *R, *b;
+  float2 *rowf, *colf;
+  int N, ky0;
+  int2 d0;
+  __device__ __forceinline__ float2 at(int rr, int k) const {
+    if (ky0 + rr >= N) return make_float2(0.f, 0.f);
+    const size_t idx = (size_t)(ky0 + rr) * N + k;
+    return cmul(cmul(cmulc(F[idx], R[idx]), rowf[rr]), colf[k % kRegK]);
+  }
+  __device__ void stage(int k0, int nk, float4* as, int pairs) const {
+    if (threadIdx.x < nk) colf[threadIdx.x] = turn_pow2(signed_freq(k0 + threadIdx.x, N) * d0.y, N);
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < pairs * kRegK; i += kRegThreads) {
+      const int p = i / kRegK, kk = i % kRegK;
+      if (kk < nk) {
+        const float2 u = at(2 * p, k0 + kk), v = at(2 * p + 1, k0 + kk);
+        as[i] = make_float4(u.x, v.x, u.y, v.y);
       }
     }
   }
-  unsigned long long mine = 0;
-  if (p < M) {
+};
+
+template <int MQ>
+__global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_rows_kernel(
+    const float2* __restrict__ F, const float2* __restrict__ Rf, const float2* __restrict__ W,
+    const unsigned long long* __restrict__ best, float2* __restrict__ T1, int N, int M) {
+  constexpr int R = reg_pairs(MQ), ROWS = reg_tile_rows(MQ);
+  extern __shared__ float4 reg_sm[];
+  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS / 2 * kRegK);
+  __shared__ float2 rowf[ROWS], colf[kRegK];
+  const int f = blockIdx.y, ky0 = blockIdx.x * ROWS;
+  const int2 d0 = coarse_shift(best[f], N);
+  for (int r = threadIdx.x; r < ROWS; r += kRegThreads)
+    rowf[r] = turn_pow2(signed_freq(ky0 + r, N) * d0.x, N);
+  float2 re[R][MQ], im[R][MQ];
+  const RegRowsSrc src{F + (size_t)f * N * N, Rf, W, rowf, colf, N, ky0, d0};
+  reg_product<MQ>(re, im, src, N, M, reg_sm, bs);
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int ky = ky0 + 2 * ((threadIdx.x / 32) * R + j);
 #pragma unroll
     for (int m = 0; m < MQ; ++m) {
-      const int q = tq + 32 * m;
-      if (q < M) {
-        const float mag = sqrtf(acc[m].x * acc[m].x + acc[m].y * acc[m].y);
-        const unsigned long long key = ((unsigned long long)__float_as_uint(mag) << 32) |
-                                       (0xffffffffu - (uint32_t)(p * M + q));
-        mine = key > mine ? key : mine;
+      const int q = threadIdx.x % 32 + 32 * m;
+      float2* t = T1 + ((size_t)f * N + ky) * M + q;
+      if (ky < N && q < M) {  // (N is even)
+        t[0] = make_float2(re[j][m].x, im[j][m].x);
+        t[M] = make_float2(re[j][m].y, im[j][m].y);
       }
+    }
+  }
+}
+
+struct RegColsSrc {
+  const float2 *W, *b;
+  int M, p0;
+  __device__ void stage(int k0, int nk, float4* as, int pairs) const {
+    const float2 zero = make_float2(0.f, 0.f);
+    for (int i = threadIdx.x; i < pairs * nk; i += kRegThreads) {
+      const int p = i % pairs, kk = i / pairs;  // neighbouring threads: neighbouring p
+      const float2* w = W + (size_t)(k0 + kk) * M + p0 + 2 * p;
+      const float2 u = p0 + 2 * p < M ? w[0] : zero, v = p0 + 2 * p + 1 < M ? w[1] : zero;
+      as[p * kRegK + kk] = make_float4(u.x, v.x, u.y, v.y);
+    }
+  }
+};
+
+template <int MQ>
+__global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_cols_kernel(
+    const float2* __restrict__ T1, const float2* __restrict__ W, int N, int M,
+    unsigned long long* __restrict__ best_up) {
+  constexpr int R = reg_pairs(MQ), ROWS = reg_tile_rows(MQ);
+  extern __shared__ float4 reg_sm[];
+  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS / 2 * kRegK);
+  const int f = blockIdx.y, p0 = blockIdx.x * ROWS;
+  float2 re[R][MQ], im[R][MQ];
+  const RegColsSrc src{W, T1 + (size_t)f * N * M, M, p0};
+  reg_product<MQ>(re, im, src, N, M, reg_sm, bs);
+  unsigned long long mine = 0;
+  auto take = [&](int p, int q, float x, float y) {
+    if (p >= M || q >= M) return;
+    const float mag = sqrtf(fmaf(x, x, y * y));  // (spelled out: near-ties turn on its last bit)
+    const unsigned long long key =
+        ((unsigned long long)__float_as_uint(mag) << 32) | (0xffffffffu - (uint32_t)(p * M + q));
+    mine = key > mine ? key : mine;
+  };
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const int p = p0 + 2 * ((threadIdx.x / 32) * R + j);
+#pragma unroll
+    for (int m = 0; m < MQ; ++m) {
+      const int q = threadIdx.x % 32 + 32 * m;
+      take(p, q, re[j][m].x, im[j][m].x);
+      take(p + 1, q, re[j][m].y, im[j][m].y);
     }
   }
 #pragma unroll
@@ -244,18 +237,36 @@ __global__ void __launch_bounds__(kRegThreads) reg_upsample_cols_kernel(
   if ((threadIdx.x & 31) == 0) atomicMax(&best_up[f], mine);
 }
 
+template <int MQ>
+static cudaError_t reg_upsample(const RegArgs& a, int N, unsigned long long* best_up, cudaStream_t st) {
+  constexpr int rows = reg_tile_rows(MQ);
+  const int smem = (int)(sizeof(float4) * rows / 2 * kRegK + sizeof(float2) * (size_t)kRegK * a.M);
+  cudaError_t e = cudaFuncSetAttribute(reg_upsample_rows_kernel<MQ>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(reg_upsample_cols_kernel<MQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  reg_upsample_rows_kernel<MQ><<<dim3((N + rows - 1) / rows, a.n), kRegThreads, smem, st>>>(
+      a.F, a.Rf, a.W, a.best, a.X, N, a.M);
+  reg_upsample_cols_kernel<MQ><<<dim3((a.M + rows - 1) / rows, a.n), kRegThreads, smem, st>>>(
+      a.X, a.W, N, a.M, best_up);
+  return cudaGetLastError();
+}
+
 // Per frame (one warp each): the refined shift d = d0 + (p* - h, q* - h)/U
 // (as the integer numerators d U), the phase of c at the peak (recomputed in
-// FP64 from T1), and the result record shifts[f] = (dy, dx, theta).
+// FP64 from T1), and the result record shifts[f] = (dy, dx, theta).  `cs`, the
+// turn e^(-i theta) that the shift applies, goes where best_up[f] was.
 __global__ void reg_finish_kernel(const float2* __restrict__ T1, const float2* __restrict__ W,
                                   const unsigned long long* __restrict__ best,
-                                  const unsigned long long* __restrict__ best_up, int n, int N,
-                                  int U, int M, int2* __restrict__ num, double* __restrict__ shifts) {
+                                  unsigned long long* best_up, int n, int N, int U, int M,
+                                  int2* __restrict__ num, double* __restrict__ shifts) {
   const int f = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   if (f >= n) return;
   const int2 d0 = coarse_shift(best[f], N);
   const uint32_t idx = 0xffffffffu - (uint32_t)(best_up[f] & 0xffffffffu);
+  float2* cs = reinterpret_cast<float2*>(best_up);
   const int p = (int)(idx / M), q = (int)(idx % M), h = M / 2;
   const float2* t1 = T1 + (long long)f * N * M;
   double re = 0.0, im = 0.0;
@@ -274,45 +285,32 @@ __global__ void reg_finish_kernel(const float2* __restrict__ T1, const float2* _
     num[f] = make_int2(ny, nx);
     shifts[3 * f] = (double)ny / U;
     shifts[3 * f + 1] = (double)nx / U;
-    shifts[3 * f + 2] = atan2(im, re);
+    const double th = atan2(im, re);
+    shifts[3 * f + 2] = th;
+    cs[f] = make_float2((float)cos(th), (float)-sin(th));  // (after the shuffles: best_up[f] is read)
   }
 }
 
-// F_f <- F_f exp(2 pi i k.d/N) exp(-i theta), d = num / U.  With
-// num = d0 U + (p - h) per axis the ramp factors into the whole-pixel turn
-// exp(2 pi i k d0 / N) and the kernel-table entry W[k][p] = exp(2 pi i k (p - h)/(U N)).
-__global__ void reg_shift_kernel(float2* __restrict__ F, int n, int N, int U, int M,
-                                 const float2* __restrict__ W, const int2* __restrict__ num,
-                                 const double* __restrict__ shifts) {
-  const long long NN = (long long)N * N, total = (long long)n * NN;
-  const int h = M / 2;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int f = (int)(k / NN);
-    const long long rem = k - f * NN;
-    const int ky = (int)(rem / N), kx = (int)(rem - (long long)ky * N);
-    const int2 d = num[f];
-    // floor division of the numerators by U: d = d0 U + (p - h), p - h in [-h, h]
-    const int d0y = (d.x + h) >= 0 ? (d.x + h) / U : -((-(d.x + h) + U - 1) / U);
-    const int d0x = (d.y + h) >= 0 ? (d.y + h) / U : -((-(d.y + h) + U - 1) / U);
-    const int py = d.x - d0y * U + h, px = d.y - d0x * U + h;
-    float2 w = turn_pow2(signed_freq(ky, N) * d0y + signed_freq(kx, N) * d0x, N);
-    w = cmul(w, cmul(W[(long long)ky * M + py], W[(long long)kx * M + px]));
-    const double th = shifts[3 * f + 2];
-    F[k] = cmul(F[k], cmul(w, make_float2((float)cos(th), (float)-sin(th))));
-  }
-}
-
-// crop the (corner) rows x cols of each N x N plane
-__global__ void reg_crop_kernel(const float2* __restrict__ src, float2* __restrict__ dst, int n,
-                                int rows, int cols, int N) {
-  const long long total = (long long)n * rows * cols;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-       k += (long long)gridDim.x * blockDim.x) {
-    const long long f = k / ((long long)rows * cols);
-    const long long rem = k - f * rows * cols;
-    const int r = (int)(rem / cols), c = (int)(rem - (long long)r * cols);
-    dst[k] = src[(f * N + r) * N + c];
+cudaError_t reg_lines(int N, int which, const RegArgs& a, cudaStream_t st) {
+  const float2* tw = nullptr;
+  cudaError_t e = twiddles(&tw);
+  if (e != cudaSuccess) return e;
+  int dev = 0, sms = 148;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  switch (N) {
+    case 8: return reg_lines_n8(which, a, tw, sms, st);
+    case 16: return reg_lines_n16(which, a, tw, sms, st);
+    case 32: return reg_lines_n32(which, a, tw, sms, st);
+    case 64: return reg_lines_n64(which, a, tw, sms, st);
+    case 128: return reg_lines_n128(which, a, tw, sms, st);
+    case 256: return reg_lines_n256(which, a, tw, sms, st);
+    case 512: return reg_lines_n512(which, a, tw, sms, st);
+    case 1024: return reg_lines_n1024(which, a, tw, sms, st);
+    case 2048: return reg_lines_n2048(which, a, tw, sms, st);
+    case 4096: return reg_lines_n4096(which, a, tw, sms, st);
+    default: return cudaErrorInvalidValue;
   }
 }
 
@@ -361,50 +359,40 @@ extern "C" int sp_register_subpixel(const void* frames_dev, int n_frames, int ro
   const RegLayout L = reg_layout(n_frames, N, upsample);
   SP_CHECK(work_bytes >= L.total, SP_ERR_WORKSPACE, "sp_register_subpixel: %zu bytes given, %zu needed",
            work_bytes, L.total);
-  const int U = upsample, M = upsampled_points(U);
   cudaStream_t st = as_stream(stream);
   char* ws = static_cast<char*>(work_dev);
-  float2* F = reinterpret_cast<float2*>(ws + L.F);
-  float2* Rf = F + (size_t)n_frames * N * N;
-  float2* X = reinterpret_cast<float2*>(ws + L.X);
-  float2* W = reinterpret_cast<float2*>(ws + L.W);
-  auto* best = reinterpret_cast<unsigned long long*>(ws + L.best);
+  const int M = upsampled_points(upsample);
   auto* best_up = reinterpret_cast<unsigned long long*>(ws + L.best_up);
+  float2* F = reinterpret_cast<float2*>(ws + L.F);
+  float2* W = reinterpret_cast<float2*>(ws + L.W);
   int2* num = reinterpret_cast<int2*>(ws + L.num);
-  const long long NN = (long long)N * N;
-  auto grid = [](long long n) { return (int)std::min<long long>((n + 255) / 256, 148LL * 16); };
-  reg_embed_kernel<<<grid(n_frames * NN), 256, 0, st>>>((const float2*)frames_dev, F, n_frames, rows,
-                                                        cols, N);
-  reg_embed_kernel<<<grid(NN), 256, 0, st>>>((const float2*)ref_dev, Rf, 1, rows, cols, N);
-  SP_CUDA_TRY(cudaGetLastError());
-  SP_CUDA_TRY(fft2_dispatch(F, F, N, n_frames + 1, 0, st));
-  reg_cross_kernel<<<grid(n_frames * NN), 256, 0, st>>>(F, Rf, X, n_frames, NN);
-  SP_CUDA_TRY(cudaGetLastError());
-  SP_CUDA_TRY(fft2_dispatch(X, X, N, n_frames, 1, st));
-  SP_CUDA_TRY(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * n_frames, st));
+  const RegArgs a{(const float2*)frames_dev, (const float2*)ref_dev, F, F + (size_t)n_frames * N * N,
+                  reinterpret_cast<float2*>(ws + L.X), W,
+                  reinterpret_cast<unsigned long long*>(ws + L.best), num,
+                  reinterpret_cast<const float2*>(best_up), (float2*)out_dev, n_frames, rows, cols,
+                  upsample, M};
+  SP_CUDA_TRY(cudaMemsetAsync(a.best, 0, sizeof(unsigned long long) * n_frames, st));
   SP_CUDA_TRY(cudaMemsetAsync(best_up, 0, sizeof(unsigned long long) * n_frames, st));
-  {
-    const int bx = (int)std::min<long long>((NN + 255) / 256, 32);
-    reg_argmax_kernel<<<dim3(bx, n_frames), 256, 0, st>>>(X, N, best);
-  }
-  reg_kernel_table<<<grid((long long)N * M), 256, 0, st>>>(W, N, U, M);
+  reg_kernel_table<<<std::min((N * M + 255) / 256, 148 * 16), 256, 0, st>>>(W, N, upsample, M);
   SP_CUDA_TRY(cudaGetLastError());
-  const size_t smem = sizeof(float2) * ((size_t)kRegRows * (kRegK + 1) + (size_t)kRegK * M);
-  SP_CUDA_TRY(cudaFuncSetAttribute(reg_upsample_rows_kernel,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  reg_upsample_rows_kernel<<<dim3((N + kRegRows - 1) / kRegRows, n_frames), kRegThreads, smem, st>>>(
-      F, Rf, W, best, X, N, M);
-  reg_upsample_cols_kernel<<<dim3((M + 7) / 8, n_frames), kRegThreads, 0, st>>>(X, W, N, M, best_up);
-  reg_finish_kernel<<<(n_frames + 3) / 4, 128, 0, st>>>(X, W, best, best_up, n_frames, N, U, M,
-                                                        num, shifts_dev);
+  for (int which : {kRegEmbed, kRegColsRef, kRegCols, kRegCross, kRegPeak})
+    SP_CUDA_TRY(reg_lines(N, which, a, st));
+  switch ((M + 31) / 32) {
+    case 1: SP_CUDA_TRY(reg_upsample<1>(a, N, best_up, st)); break;
+    case 2: SP_CUDA_TRY(reg_upsample<2>(a, N, best_up, st)); break;
+    case 3: SP_CUDA_TRY(reg_upsample<3>(a, N, best_up, st)); break;
+    case 4: SP_CUDA_TRY(reg_upsample<4>(a, N, best_up, st)); break;
+    case 5: SP_CUDA_TRY(reg_upsample<5>(a, N, best_up, st)); break;
+    case 6: SP_CUDA_TRY(reg_upsample<6>(a, N, best_up, st)); break;
+    case 7: SP_CUDA_TRY(reg_upsample<7>(a, N, best_up, st)); break;
+    default: SP_CUDA_TRY(reg_upsample<8>(a, N, best_up, st)); break;
+  }
+  reg_finish_kernel<<<(n_frames + 3) / 4, 128, 0, st>>>(a.X, W, a.best, best_up, n_frames, N, upsample,
+                                                        M, num, shifts_dev);
   SP_CUDA_TRY(cudaGetLastError());
   if (out_dev) {
-    reg_shift_kernel<<<grid(n_frames * NN), 256, 0, st>>>(F, n_frames, N, U, M, W, num, shifts_dev);
-    SP_CUDA_TRY(cudaGetLastError());
-    SP_CUDA_TRY(fft2_dispatch(F, F, N, n_frames, 1, st));  // inverse, scaled by 1/N^2
-    reg_crop_kernel<<<grid((long long)n_frames * rows * cols), 256, 0, st>>>(F, (float2*)out_dev,
-                                                                            n_frames, rows, cols, N);
-    SP_CUDA_TRY(cudaGetLastError());
+    SP_CUDA_TRY(reg_lines(N, kRegShift, a, st));
+    SP_CUDA_TRY(reg_lines(N, kRegCrop, a, st));
   }
   return SP_OK;
 }
