@@ -90,6 +90,8 @@ _SIGS = {
     "sp_align_global_phase": ([_p, _i, _i64, _p, _p, _p], _i),
     "sp_prtf": ([_p, _i, _i, _i, _i, _p, _p, _p], _i),
     "sp_shrinkwrap": ([_p, _i, _i, _p, _p, _p, _i, _d, _d, _i, _p, _p, _p, _p, _p], _i),
+    "sp_refine_workspace_size": ([_i, _i, C.POINTER(_sz)], _i),
+    "sp_refine_support": ([_p, _i, _i, _p, _p, _p, _d, _d, _i, _p, _sz, _p, _p, _p], _i),
     "sp_mean_frames": ([_p, _i, _i64, _p, _p], _i),
     "sp_prtf_phasors": ([_p, _i, _i, _i, _i, _p, _p, _p], _i),
     "sp_prtf_finish": ([_p, _i, _i, _p, _p], _i),

@@ -1,10 +1,9 @@
 // Operator API (one entry per reference OpenCL kernel), the standalone 2-D
 // FFT entry point, and the post-processing kernels of the phasing path:
-// global-phase alignment, PRTF, shrinkwrap blur/threshold, averaging and the
-// cross-correlation peak used by integer frame alignment.
+// global-phase alignment, PRTF, averaging and the cross-correlation peak used
+// by integer frame alignment.
 #include <cmath>
 #include <cstring>
-#include <vector>
 
 #include "sp_common.cuh"
 #include "sp_fft2.cuh"
@@ -281,88 +280,6 @@ __global__ void mean_frames_kernel(const float2* __restrict__ frames, int n, int
 }
 
 // ---------------------------------------------------------------------------
-// shrinkwrap: separable circular Gaussian blur of |avg| in FP64
-// (phasing.py:1786-1790: ifft2(fft2(fftshift(g)/sum g) * fft2(|avg|)).real is a
-// circular convolution with the separable kernel k_r (x) k_c), then thresholds
-// ---------------------------------------------------------------------------
-__global__ void blur_rows_kernel(const float2* __restrict__ avg, const double* __restrict__ kc,
-                                 double* __restrict__ tmp, int rows, int cols) {
-  const int64_t total = (int64_t)rows * cols;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(k / cols), c = (int)(k - (int64_t)r * cols);
-    double s = 0;
-    for (int j = 0; j < cols; ++j) {
-      int cc = c - j;
-      if (cc < 0) cc += cols;
-      const float2 v = avg[(int64_t)r * cols + cc];
-      s = fma(kc[j], (double)sqrtf(v.x * v.x + v.y * v.y), s);
-    }
-    tmp[k] = s;
-  }
-}
-__global__ void blur_cols_kernel(const double* __restrict__ tmp, const double* __restrict__ kr,
-                                 double* __restrict__ blurred, int rows, int cols) {
-  const int64_t total = (int64_t)rows * cols;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(k / cols), c = (int)(k - (int64_t)r * cols);
-    double s = 0;
-    for (int i = 0; i < rows; ++i) {
-      int rr = r - i;
-      if (rr < 0) rr += rows;
-      s = fma(kr[i], tmp[(int64_t)rr * cols + c], s);
-    }
-    blurred[k] = s;
-  }
-}
-// per-label maxima of blurred and sums of |avg| (label 0 = global max), as
-// order-preserving 64-bit keys for atomicMax
-__device__ __forceinline__ unsigned long long dkey(double x) {
-  unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double dkey_inv(unsigned long long k) {
-  const unsigned long long u = (k & 0x8000000000000000ull) ? (k & ~0x8000000000000000ull) : ~k;
-  return __longlong_as_double((long long)u);
-}
-__global__ void label_stats_kernel(const double* __restrict__ blurred, const float2* __restrict__ avg,
-                                   const int* __restrict__ labels, int64_t total,
-                                   unsigned long long* __restrict__ maxkey, double* __restrict__ sums) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const double b = blurred[k];
-    atomicMax(&maxkey[0], dkey(b));
-    const int l = labels ? labels[k] : 0;
-    if (l > 0) {
-      atomicMax(&maxkey[l], dkey(b));
-      const float2 v = avg[k];
-      atomicAdd(&sums[l], (double)sqrtf(v.x * v.x + v.y * v.y));
-    }
-  }
-}
-// refined = sum over parts of (b*part > max(b*part)*lt) times (b > max(b)*gt)
-__global__ void threshold_kernel(const double* __restrict__ blurred, const int* __restrict__ labels,
-                                 int64_t total, const unsigned long long* __restrict__ maxkey,
-                                 double local_t, double global_t, int kill_label,
-                                 float* __restrict__ refined) {
-  const double gmax = dkey_inv(maxkey[0]);
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const double b = blurred[k];
-    const int l = labels[k];
-    float r = 0.f;
-    if (l > 0 && l != kill_label) {
-      // current.max() over the whole array includes the zeros outside the part
-      const double pmax = fmax(dkey_inv(maxkey[l]), 0.0);
-      r = (b > pmax * local_t) ? 1.f : 0.f;
-    }
-    if (!(b > gmax * global_t)) r = 0.f;
-    refined[k] = r;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // cross-correlation peak: argmax over the fftshifted |cc| (crosscorr.py:556)
 // keyed so that ties go to the first index in shifted order, as numpy's argmax
 // ---------------------------------------------------------------------------
@@ -622,42 +539,6 @@ int sp_mean_frames(const void* frames, int n_frames, int64_t frame_elems, void* 
            "sp_mean_frames: bad argument");
   mean_frames_kernel<<<grid_for(frame_elems), 256, 0, as_stream(stream)>>>(
       (const float2*)frames, n_frames, frame_elems, (float2*)out);
-  SP_CUDA_TRY(cudaGetLastError());
-  return SP_OK;
-}
-
-int sp_shrinkwrap(const void* avg, int rows, int cols, const double* kr, const double* kc,
-                  const int* labels, int n_labels, double local_t, double global_t, int kill_weakest,
-                  void* work, double* blurred, float* refined, double* part_sums,
-                  sp_stream_t stream) {
-  SP_CHECK(avg && kr && kc && labels && work && blurred && refined && part_sums, SP_ERR_INVALID,
-           "sp_shrinkwrap: null pointer");
-  SP_CHECK(rows > 0 && cols > 0 && n_labels >= 0, SP_ERR_INVALID, "sp_shrinkwrap: bad size");
-  cudaStream_t st = as_stream(stream);
-  const int64_t total = (int64_t)rows * cols;
-  double* tmp = static_cast<double*>(work);
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(tmp + total);
-  blur_rows_kernel<<<grid_for(total), 256, 0, st>>>((const float2*)avg, kc, tmp, rows, cols);
-  blur_cols_kernel<<<grid_for(total), 256, 0, st>>>(tmp, kr, blurred, rows, cols);
-  // keys start at the smallest order-preserving key (0 encodes -NaN, below all)
-  SP_CUDA_TRY(cudaMemsetAsync(keys, 0, sizeof(unsigned long long) * (n_labels + 1), st));
-  SP_CUDA_TRY(cudaMemsetAsync(part_sums, 0, sizeof(double) * (n_labels + 1), st));
-  label_stats_kernel<<<grid_for(total), 256, 0, st>>>(blurred, (const float2*)avg, labels, total,
-                                                      keys, part_sums);
-  SP_CUDA_TRY(cudaGetLastError());
-  int kill = -1;
-  if (kill_weakest && n_labels > 0) {
-    // the weakest part is chosen on the host from part_sums (phasing.py:1811-1813)
-    std::vector<double> h(n_labels + 1);
-    SP_CUDA_TRY(cudaMemcpyAsync(h.data(), part_sums, sizeof(double) * (n_labels + 1),
-                                cudaMemcpyDeviceToHost, st));
-    SP_CUDA_TRY(cudaStreamSynchronize(st));
-    kill = 1;
-    for (int l = 2; l <= n_labels; ++l)
-      if (h[l] < h[kill]) kill = l;
-  }
-  threshold_kernel<<<grid_for(total), 256, 0, st>>>(blurred, labels, total, keys, local_t, global_t,
-                                                    kill, refined);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }

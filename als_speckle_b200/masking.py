@@ -58,7 +58,16 @@ def bounding_box(data, threshold=1e-10, force_to_square=False, pad=0):
     return np.array([rmin, rmax, cmin, cmax]).astype(int)
 
 
-def label_parts(data, detect_val=(0.95, 1.05)):
+DETECT = (0.95, 1.05)  # support values that count as inside
+
+
+def inside(data, detect_val=DETECT):
+    """Mask of the (nearly binary) support's inside, as ``label_parts`` uses it."""
+    data = np.asarray(data)
+    return (data >= detect_val[0]) & (data <= detect_val[1])
+
+
+def label_parts(data, detect_val=DETECT):
     """Connected parts of a (nearly binary) support, numbered 1..n.
 
     Connectivity is 8-neighbour with periodic wrap and parts are numbered in
@@ -68,8 +77,7 @@ def label_parts(data, detect_val=(0.95, 1.05)):
     n counts empty parts (isolated pixels), whose label has no pixels.
     """
     from scipy import ndimage
-    data = np.asarray(data)
-    mask = (data >= detect_val[0]) & (data <= detect_val[1])
+    mask = inside(data, detect_val)
     R, C = mask.shape
     lab, n = ndimage.label(mask, structure=np.ones((3, 3), bool))
     if n == 0:

@@ -658,16 +658,16 @@ def refine_support(support, average_mag, blur=3, local_threshold=.2, global_thre
         raise ValueError("support and average_mag must have the same shape")
     dev = avg_t.device
     kr = torch.from_numpy(_gaussian_1d_kernel(rows, blur)).to(dev)
-    kc = torch.from_numpy(_gaussian_1d_kernel(cols, blur)).to(dev)
-    labels, n = masking.label_parts(support)
-    lab = torch.from_numpy(labels.astype(np.int32)).to(dev)
-    work = torch.empty(rows * cols + n + 1, dtype=torch.float64, device=dev)
+    kc = kr if rows == cols else torch.from_numpy(_gaussian_1d_kernel(cols, blur)).to(dev)
+    mask = torch.from_numpy(np.ascontiguousarray(masking.inside(support)).view(np.uint8)).to(dev)
+    nbytes = C.c_size_t(0)
+    call("sp_refine_workspace_size", rows, cols, C.byref(nbytes))
+    work = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
     blurred = torch.empty((rows, cols), dtype=torch.float64, device=dev)
     refined = torch.empty((rows, cols), dtype=torch.float32, device=dev)
-    sums = torch.empty(n + 1, dtype=torch.float64, device=dev)
-    call("sp_shrinkwrap", ptr(avg_t), rows, cols, ptr(kr), ptr(kc), ptr(lab), n,
-         float(local_threshold), float(global_threshold), 1 if kill_weakest else 0,
-         ptr(work), ptr(blurred), ptr(refined), ptr(sums), stream_ptr())
+    call("sp_refine_support", ptr(avg_t), rows, cols, ptr(kr), ptr(kc), ptr(mask),
+         float(local_threshold), float(global_threshold), 1 if kill_weakest else 0, ptr(work),
+         nbytes.value, ptr(blurred), ptr(refined), stream_ptr())
     ref = refined.cpu().numpy().astype(support.dtype if support.dtype.kind == "f" else np.int64)
     return ref, blurred.cpu().numpy()
 

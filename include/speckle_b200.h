@@ -209,6 +209,15 @@ int sp_shrinkwrap(const void* avg_dev, int rows, int cols, const double* kr_dev,
                   const double* kc_dev, const int* labels_dev, int n_labels, double local_t,
                   double global_t, int kill_weakest, void* work_dev, double* blurred_dev,
                   float* refined_dev, double* part_sums_dev, sp_stream_t stream);
+/* The same with the parts found on the device: mask_dev (bytes, rows*cols, non-zero
+ * inside the support) is split into its connected parts (8 neighbours, periodic; a
+ * pixel with no neighbour in the mask is an empty part).  work_dev: scratch of
+ * sp_refine_workspace_size bytes, 8-byte aligned. */
+int sp_refine_workspace_size(int rows, int cols, size_t* bytes);
+int sp_refine_support(const void* avg_dev, int rows, int cols, const double* kr_dev,
+                      const double* kc_dev, const unsigned char* mask_dev, double local_t,
+                      double global_t, int kill_weakest, void* work_dev, size_t work_bytes,
+                      double* blurred_dev, float* refined_dev, sp_stream_t stream);
 /* Average of aligned frames (basic_phasing_example.py:43): out = mean over n. */
 int sp_mean_frames(const void* frames_dev, int n_frames, int64_t frame_elems, void* out_dev,
                    sp_stream_t stream);
