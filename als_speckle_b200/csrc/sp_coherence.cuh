@@ -46,6 +46,19 @@ __host__ __device__ constexpr int pc_smem_elems() {
   return item_smem_elems(N, pc_e(N)) + tw_stage_total(N, pc_e(N));
 }
 
+// Up to 512^2 the column and row kernels are launched programmatically, as the
+// pass kernels are (see pdl_allow_next); above, where a plane alone fills the
+// chip, that measured slower (2 trials of 2048^2 with an ipsf: 509 against 446 us
+// per iteration).
+__host__ __device__ constexpr bool pc_programmatic(int N) { return N <= 512; }
+template <int N>
+__device__ __forceinline__ void pc_chain() {
+  if constexpr (pc_programmatic(N)) {
+    pdl_wait_prev();
+    pdl_allow_next();
+  }
+}
+
 // A: F = FFT_cols(G) over G, W = FFT_cols(|F|^2).
 template <int N>
 __global__ void __launch_bounds__(kThreads, 4) pc_cols_a_kernel(PcArgs a) {
@@ -57,6 +70,7 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_a_kernel(PcArgs a) {
   const bool active = t < T;
   const ColLayout<pad_shift(E), C> lay{smem + c};
   constexpr int PER = N / C;
+  pc_chain<N>();  // the planes are earlier kernels' output
   for (int it = blockIdx.x; it < a.n_jobs * PER; it += gridDim.x) {
     const int j = it / PER, blk = it - j * PER;
     const int2 job = a.jobs[j];
@@ -97,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_a_kernel(PcArgs a) {
 
 // W: W = IFFT_rows(FFT_rows(W) * ipsf), unnormalised.
 template <int N>
-__global__ void __launch_bounds__(kThreads) pc_rows_w_kernel(PcArgs a) {
+__global__ void __launch_bounds__(kThreads, N <= 512 ? 4 : 3) pc_rows_w_kernel(PcArgs a) {
   constexpr int E = pc_e(N), T = N / E, L = lines_per_item(N, E), SH = pad_shift(E);
   using Sync = typename std::conditional<(T <= 32), WarpSync, BlockSync>::type;
   extern __shared__ float2 smem[];
@@ -109,6 +123,7 @@ __global__ void __launch_bounds__(kThreads) pc_rows_w_kernel(PcArgs a) {
   const int lr = active ? lrow : 0;
   const RowLayout<SH> lay{smem + lr * padk(N, SH)};
   constexpr int PER = N / L;
+  pc_chain<N>();
   for (int it = blockIdx.x; it < a.n_jobs * PER; it += gridDim.x) {
     const int j = it / PER, blk = it - j * PER;
     const int2 job = a.jobs[j];
@@ -147,6 +162,7 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_b_kernel(PcArgs a) {
   const bool active = t < T;
   const ColLayout<pad_shift(E), C> lay{smem + c};
   constexpr int PER = N / C;
+  pc_chain<N>();  // the planes are earlier kernels' output
   for (int it = blockIdx.x; it < a.n_jobs * PER; it += gridDim.x) {
     const int j = it / PER, blk = it - j * PER;
     const int2 job = a.jobs[j];
@@ -232,6 +248,7 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_b1_kernel(PcArgs a) {
   const bool active = t < T;
   const ColLayout<pad_shift(E), C> lay{smem + c};
   constexpr int PER = N / C;
+  pc_chain<N>();  // the planes are earlier kernels' output
   for (int it = blockIdx.x; it < a.n_jobs * PER; it += gridDim.x) {
     const int j = it / PER, blk = it - j * PER;
     const int2 job = a.jobs[j];
@@ -268,8 +285,13 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_b1_kernel(PcArgs a) {
 // tile of TC columns x RB rows; each thread owns one column and RT of the
 // tile's rows.  The row taps of up to RQ samples (their weights times w_k)
 // are built once per tile in shared memory, a thread's column taps in
-// registers, so a sample costs a pixel four loads and four FMAs:
+// registers, so a sample costs a pixel four FMAs and, each source row being
+// interpolated across once for the two output rows it serves, little over two
+// loads:
 //   out += (w_k wy1) (v11 wx1 + v21 wx2) + (w_k wy2) (v12 wx1 + v22 wx2).
+// Bound by L1, issue and load latency (four loads a sample and pixel: 38 us for
+// 16 planes of 512^2 and seven samples, L1 wavefronts 66% and issue 57% of their
+// peaks; now 32 us), so a thread issues the loads of four rows together.
 struct RescaleTap {
   int i1, i2;    // source index of each tap (column, or row * N); 0 where the weight is 0
   float w1, w2;  // 1 - |tap - r| (times the spectral weight for rows)
@@ -307,7 +329,7 @@ __device__ __forceinline__ RescaleTap rescale_tap(int N, float c, float r, int s
 }
 
 template <int N>
-__global__ void __launch_bounds__(kThreads, 5) pc_rescale_kernel(PcArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) pc_rescale_kernel(PcArgs a) {
   using RT_ = RescaleTile<N>;
   constexpr int TC = RT_::TC, G = RT_::G, RB = RT_::RB, RT = RT_::RT, RQ = RT_::RQ;
   constexpr int N2 = N / 2;
@@ -340,41 +362,83 @@ __global__ void __launch_bounds__(kThreads, 5) pc_rescale_kernel(PcArgs a) {
       __syncthreads();
       for (int q = 0; q < nq; ++q) {
         const RescaleTap x = rescale_tap(N, xc, rq[q], 1, 1.f);
+        // a row's second source row is nearly always the next row's first (the
+        // samples stretch the plane by a few percent), so each source row is
+        // interpolated once; the taps are the same for a whole warp
+        constexpr int B = RT < 4 ? RT : 4;  // rows whose loads are issued together
+        int have = -1;
+        float h = 0.f;
 #pragma unroll
-        for (int u = 0; u < RT; ++u) {
-          const int lr = g + u * G;
-          if (RB % G == 0 || lr < RB) {
-            const RescaleTap y = yt[q][lr];
-            const float h1 = fmaf(pp[y.i1 + x.i2], x.w2, pp[y.i1 + x.i1] * x.w1);
-            const float h2 = fmaf(pp[y.i2 + x.i2], x.w2, pp[y.i2 + x.i1] * x.w1);
-            cum[u] = fmaf(y.w2, h2, fmaf(y.w1, h1, cum[u]));
+        for (int u0 = 0; u0 < RT; u0 += B) {
+          RescaleTap y[B];
+          float p1[B], p2[B], q1[B], q2[B];
+#pragma unroll
+          for (int u = 0; u < B; ++u) {
+            const int lr = g * RT + u0 + u;
+            y[u] = yt[q][RB % G == 0 || lr < RB ? lr : 0];
+            p1[u] = pp[y[u].i2 + x.i1];
+            p2[u] = pp[y[u].i2 + x.i2];
+          }
+#pragma unroll
+          for (int u = 0; u < B; ++u) {
+            const bool fresh = y[u].i1 != (u ? y[u - 1].i2 : have);
+            q1[u] = fresh ? pp[y[u].i1 + x.i1] : 0.f;
+            q2[u] = fresh ? pp[y[u].i1 + x.i2] : 0.f;
+          }
+#pragma unroll
+          for (int u = 0; u < B; ++u) {
+            const bool fresh = y[u].i1 != have;
+            const float h1 = fresh ? fmaf(q2[u], x.w2, q1[u] * x.w1) : h;
+            h = fmaf(p2[u], x.w2, p1[u] * x.w1);
+            have = y[u].i2;
+            cum[u0 + u] = fmaf(y[u].w2, h, fmaf(y[u].w1, h1, cum[u0 + u]));
           }
         }
       }
     }
 #pragma unroll
     for (int u = 0; u < RT; ++u) {
-      const int lr = g + u * G;
+      const int lr = g * RT + u;
       if (RB % G == 0 || lr < RB) out[(int64_t)(r0 + lr) * N + col] = cum[u];
     }
   }
 }
 
-// which: 0 = A, 1 = W, 2 = B1, 3 = R, 4 = B
+// Dynamic shared memory of a column or row kernel with `per_sm` CTAs for every
+// SM: padded so that no more than these fit.  The kernels are let in while the
+// previous one drains (pdl_allow_next), and with room for four everywhere a
+// grid of fewer would pile up on the SMs that drain first (4 trials of 512^2
+// with an ipsf: 44 us per iteration, 35 padded, 38 with plain launches; 32
+// trials 190, 197 with plain launches; one trial 25 and 29).
 template <int N>
-cudaError_t launch_pc_t(int which, int grid, cudaStream_t st, const PcArgs& a) {
-  const size_t sm = (size_t)pc_smem_elems<N>() * sizeof(float2);
-  if (which == 0) pc_cols_a_kernel<N><<<grid, kThreads, sm, st>>>(a);
-  else if (which == 1) pc_rows_w_kernel<N><<<grid, kThreads, sm, st>>>(a);
-  else if (which == 2) pc_cols_b1_kernel<N><<<grid, kThreads, sm, st>>>(a);
-  else if (which == 3) pc_rescale_kernel<N><<<grid, kThreads, 0, st>>>(a);
-  else pc_cols_b_kernel<N><<<grid, kThreads, sm, st>>>(a);
+size_t pc_smem_bytes(int per_sm) {
+  const size_t need = (size_t)pc_smem_elems<N>() * sizeof(float2);
+  if (per_sm >= 4) return need;
+  const size_t room = (size_t)(228 * 1024 / per_sm - 1024) / 1024 * 1024;  // 1 KB per CTA is reserved
+  return room > need ? room : need;
+}
+
+// which: 0 = A, 1 = W, 2 = B1, 3 = R, 4 = B.  R keeps a plain launch: it lives on
+// L1 hits, which padding would cost.
+template <int N>
+cudaError_t launch_pc_t(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) {
+  if (which == 3) {
+    pc_rescale_kernel<N><<<grid, kThreads, 0, st>>>(a);
+    return cudaGetLastError();
+  }
+  void (*k)(PcArgs) = which == 0   ? pc_cols_a_kernel<N>
+                      : which == 1 ? pc_rows_w_kernel<N>
+                      : which == 2 ? pc_cols_b1_kernel<N>
+                                   : pc_cols_b_kernel<N>;
+  if constexpr (pc_programmatic(N))
+    return launch_pdl(k, grid, kThreads, pc_smem_bytes<N>((grid + n_sms - 1) / n_sms), st, a);
+  k<<<grid, kThreads, pc_smem_bytes<N>(4), st>>>(a);
   return cudaGetLastError();
 }
 
 template <int N>
 cudaError_t pc_setup_t() {
-  const int sm = pc_smem_elems<N>() * (int)sizeof(float2);
+  const int sm = (int)pc_smem_bytes<N>(1);
   cudaError_t e = cudaFuncSetAttribute(pc_cols_a_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(pc_rows_w_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -392,7 +456,7 @@ constexpr int pc_items_per_job() { return N / lines_per_item(N, pc_e(N)); }
 
 namespace sp {
 #define SP_DECLARE_PC(N)                                                              \
-  cudaError_t launch_pc_n##N(int which, int grid, cudaStream_t st, const PcArgs& a); \
+  cudaError_t launch_pc_n##N(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a); \
   cudaError_t pc_setup_n##N();
 SP_DECLARE_PC(8)
 SP_DECLARE_PC(16)
@@ -406,8 +470,8 @@ SP_DECLARE_PC(2048)
 SP_DECLARE_PC(4096)
 
 #define SP_DEFINE_PC(N)                                                                \
-  cudaError_t launch_pc_n##N(int which, int grid, cudaStream_t st, const PcArgs& a) { \
-    return launch_pc_t<N>(which, grid, st, a);                                        \
+  cudaError_t launch_pc_n##N(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) { \
+    return launch_pc_t<N>(which, grid, n_sms, st, a);                                        \
   }                                                                                    \
   cudaError_t pc_setup_n##N() { return pc_setup_t<N>(); }
 }  // namespace sp

@@ -53,18 +53,18 @@ static cudaError_t pass_setup(int N, int E, int* occ) {
   }
 }
 
-static cudaError_t launch_pc(int N, int which, int grid, cudaStream_t st, const PcArgs& a) {
+static cudaError_t launch_pc(int N, int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) {
   switch (N) {
-    case 8: return launch_pc_n8(which, grid, st, a);
-    case 16: return launch_pc_n16(which, grid, st, a);
-    case 32: return launch_pc_n32(which, grid, st, a);
-    case 64: return launch_pc_n64(which, grid, st, a);
-    case 128: return launch_pc_n128(which, grid, st, a);
-    case 256: return launch_pc_n256(which, grid, st, a);
-    case 512: return launch_pc_n512(which, grid, st, a);
-    case 1024: return launch_pc_n1024(which, grid, st, a);
-    case 2048: return launch_pc_n2048(which, grid, st, a);
-    case 4096: return launch_pc_n4096(which, grid, st, a);
+    case 8: return launch_pc_n8(which, grid, n_sms, st, a);
+    case 16: return launch_pc_n16(which, grid, n_sms, st, a);
+    case 32: return launch_pc_n32(which, grid, n_sms, st, a);
+    case 64: return launch_pc_n64(which, grid, n_sms, st, a);
+    case 128: return launch_pc_n128(which, grid, n_sms, st, a);
+    case 256: return launch_pc_n256(which, grid, n_sms, st, a);
+    case 512: return launch_pc_n512(which, grid, n_sms, st, a);
+    case 1024: return launch_pc_n1024(which, grid, n_sms, st, a);
+    case 2048: return launch_pc_n2048(which, grid, n_sms, st, a);
+    case 4096: return launch_pc_n4096(which, grid, n_sms, st, a);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -307,6 +307,7 @@ struct Segment {
   int pc_egrid;                     // grid of the tiled rescale kernel
   int col_ticks;                    // the column pass runs at ticks [0, col_ticks)
   int pc_mask;                      // partial-coherence kernels launched (bit = which)
+  int sms;                          // of the device
   int ticks;                        // ticks of this segment's longest trial (n_iter + 1)
 };
 
@@ -333,7 +334,7 @@ static int launch_segment(const Segment& sg, const Slot* slots, const Item* item
       PcArgs pa{slots, jobs + sg.pc_first, sg.pc_count, k, tw};
       for (int which = 0; which < 5; ++which)
         if (sg.pc_mask & (1 << which))
-          SP_CUDA_TRY(launch_pc(sg.N, which, which == 3 ? sg.pc_egrid : sg.pc_grid, st, pa));
+          SP_CUDA_TRY(launch_pc(sg.N, which, which == 3 ? sg.pc_egrid : sg.pc_grid, sg.sms, st, pa));
     }
     for (int which = 0; which < 2; ++which) {
       if (which == 0 && k >= sg.col_ticks) continue;  // no column work left in this segment
@@ -501,7 +502,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       if (count == 0) continue;
       int occ[kPassKinds], sms = 1;
       SP_CUDA_TRY(occupancy_for(N, E, occ, &sms));
-      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, 0};
+      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, sms, 0};
       for (int i = gstart[g]; i < gstart[g + 1]; ++i)
         if (trials[i].n == N) sg.ticks = std::max(sg.ticks, trials[i].n_iter + 1);
       // Partially coherent slots project in their own kernels: the column
@@ -534,7 +535,11 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       if (sg.pc_count > 0) {
         SP_CUDA_TRY(pc_ready(N));
         const int per_job = N / lines_per_item(N, pc_e(N));
-        sg.pc_grid = std::max(1, std::min(sg.pc_count * per_job, sms * 4));
+        // up to 512^2 a CTA for every item (the hardware deals the uneven last
+        // round out: 2-5% on 16-45 trials); above, persistent CTAs, whose
+        // larger twiddle tables are worth keeping
+        const int64_t units = (int64_t)sg.pc_count * per_job;
+        sg.pc_grid = (int)std::max<int64_t>(1, N <= 512 ? units : std::min<int64_t>(units, sms * 4));
         const int64_t tiles = (int64_t)sg.pc_count * N * N / rescale_tile_pixels(N);
         sg.pc_egrid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 8));
       }
