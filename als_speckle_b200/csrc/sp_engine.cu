@@ -308,6 +308,8 @@ struct Segment {
   int col_ticks;                    // the column pass runs at ticks [0, col_ticks)
   int pc_mask;                      // partial-coherence kernels launched (bit = which)
   int sms;                          // of the device
+  double rounds;                    // of the SMs that a row pass takes
+  double work;                      // pixels times projections of a tick
   int ticks;                        // ticks of this segment's longest trial (n_iter + 1)
 };
 
@@ -323,30 +325,6 @@ struct GraphKey {
 static std::mutex g_graph_mutex;
 static std::map<GraphKey, cudaGraphExec_t> g_graphs;
 static thread_local int64_t g_last_launches = 0;
-
-// One segment's launch chain: per tick its partial-coherence kernels, its
-// column pass and its row pass.
-static int launch_segment(const Segment& sg, const Slot* slots, const Item* items,
-                          const int2* jobs, const float2* tw, cudaStream_t st) {
-  for (int k = 0; k < sg.ticks; ++k) {
-    // partially coherent projections first (their slots sit out the column pass)
-    if (sg.pc_count > 0) {
-      PcArgs pa{slots, jobs + sg.pc_first, sg.pc_count, k, tw};
-      for (int which = 0; which < 5; ++which)
-        if (sg.pc_mask & (1 << which))
-          SP_CUDA_TRY(launch_pc(sg.N, which, which == 3 ? sg.pc_egrid : sg.pc_grid, sg.sms, st, pa));
-    }
-    for (int which = 0; which < 2; ++which) {
-      if (which == 0 && k >= sg.col_ticks) continue;  // no column work left in this segment
-      // the column pass walks the items backwards: it starts on the trials
-      // whose G planes the row pass wrote last (still in L2), and the next
-      // row pass starts on the ones it wrote last
-      PassArgs a{slots, items + sg.first, sg.count, nullptr, k, tw, which == 0 ? 1 : 0};
-      SP_CUDA_TRY(launch_pass(sg.N, sg.E, sg.kind[which], sg.grid[which], st, a));
-    }
-  }
-  return SP_OK;
-}
 
 // Auxiliary streams and events of the calling thread, per device, for the
 // concurrent segment chains (created before any capture begins), released
@@ -386,42 +364,96 @@ static cudaError_t fork_pool(int dev, int branches, ForkPool** out) {
   return cudaSuccess;
 }
 
-// Every segment of a group, each as its own chain: segments share no data
-// (their trials, planes and items are disjoint; slots, items and transposed
-// moduli are only read), so the chains of different sizes run concurrently
-// -- the first on `st`, the others on auxiliary streams forked from it and
-// joined back into it (in a capture this forms parallel graph branches).  The
-// joins are made even after a failed launch, so a capture never ends with
-// unjoined work.
+// The launches of several sizes in one stream: per tick the partial-coherence
+// kernels and column passes of every size, then their row passes.  Sizes share
+// no data (their trials, planes and items are disjoint; slots, items and
+// transposed moduli are only read), so a pass that follows one of another size
+// starts on the SMs that one's last round leaves idle (PassArgs.overlap).
+// `beside`: other lines run concurrently (PassArgs.late).
+static int launch_line(const std::vector<Segment>& segs, const Slot* slots, const Item* items,
+                       const int2* jobs, const float2* tw, bool beside, cudaStream_t st) {
+  int ticks = 0;
+  for (const Segment& sg : segs) ticks = std::max(ticks, sg.ticks);
+  int prev = -1;  // segment of the previous launch
+  for (int k = 0; k < ticks; ++k) {
+    for (int which = 0; which < 2; ++which) {
+      for (int i = 0; i < (int)segs.size(); ++i) {
+        const Segment& sg = segs[i];
+        if (k >= sg.ticks) continue;
+        if (which == 0) {
+          // partially coherent projections (their slots sit out the column pass)
+          if (sg.pc_count > 0) {
+            PcArgs pa{slots, jobs + sg.pc_first, sg.pc_count, k, tw};
+            for (int w = 0; w < 5; ++w)
+              if (sg.pc_mask & (1 << w))
+                SP_CUDA_TRY(launch_pc(sg.N, w, w == 3 ? sg.pc_egrid : sg.pc_grid, sg.sms, st, pa));
+            prev = i;
+          }
+          if (k >= sg.col_ticks) continue;  // no column work left in this segment
+        }
+        // the column pass walks the items backwards: it starts on the trials
+        // whose G planes the row pass wrote last (still in L2), and the next
+        // row pass starts on the ones it wrote last
+        const bool overlap = prev >= 0 && prev != i && sg.pc_count == 0 && sg.kind[which] <= kPassRow;
+        const bool in_line = (segs.size() > 1 || beside) && sg.kind[which] <= kPassRow;
+        const int kind = in_line ? sg.kind[which] + kPassColLine : sg.kind[which];
+        PassArgs a{slots, items + sg.first, sg.count, nullptr, k, tw, which == 0 ? 1 : 0, overlap, beside};
+        SP_CUDA_TRY(launch_pass(sg.N, sg.E, kind, sg.grid[which], st, a));
+        prev = i;
+      }
+    }
+  }
+  return SP_OK;
+}
+
+// Every segment of a group.  The sizes whose passes take more than one round of
+// the SMs share one line of launches; a size that leaves SMs idle gets its own,
+// on an auxiliary stream forked from `st` and joined back into it (in a capture
+// this forms parallel graph branches), unless it nearly fills them and is a
+// small part of the work.  Lines that all fill the chip get in one another's
+// way: waiting CTAs of one hold SMs that another could use.  us per iteration
+// with a line per size / as here: 64 x 256^2 + 32 x 512^2 + 8 x 1024^2 + 2 x 2048^2
+// 460 / 402; 16 x 512^2 + 4 x 1024^2 136 / 118; 16 x 256^2 + 8 x 512^2 + 3 x 1024^2 +
+// 2048^2 245 / 201 alone, 219 / 176 with calls on three streams (the 256^2
+// trials in a line of their own: 187 and 210).  Everything in one line is slower
+// where sizes leave SMs idle (512^2 + 1024^2: 29 / 34).  The joins are made even
+// after a failed launch, so a capture never ends with unjoined work.
 static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, const Item* items,
                         const int2* jobs, const float2* tw, ForkPool* P, cudaStream_t st) {
-  if (segs.size() == 1 || P == nullptr) {
-    for (const Segment& sg : segs) {
-      const int rc = launch_segment(sg, slots, items, jobs, tw, st);
-      if (rc != SP_OK) return rc;
-    }
-    return SP_OK;
+  if (P == nullptr || segs.size() == 1)
+    return launch_line(segs, slots, items, jobs, tw, false, st);
+  double work = 0;
+  for (const Segment& sg : segs) work += sg.work;
+  auto shared = [&](const Segment& sg) {
+    return sg.rounds > 1.0 || (sg.rounds > 0.75 && sg.work < 0.2 * work);
+  };
+  std::vector<std::vector<Segment>> lines(1);  // [0] on `st`
+  for (const Segment& sg : segs)
+    if (shared(sg)) lines[0].push_back(sg);
+  for (const Segment& sg : segs) {
+    if (shared(sg)) continue;
+    if (lines[0].empty()) lines[0].push_back(sg);
+    else lines.push_back({sg});
   }
-  const int n_aux = (int)segs.size() - 1;
+  const int n_aux = (int)lines.size() - 1;
   SP_CUDA_TRY(cudaEventRecord(P->events[0], st));
   int rc = SP_OK;
   int forked = 0;
   for (int i = 0; i < n_aux; ++i) {
     if (cudaStreamWaitEvent(P->streams[i], P->events[0], 0) != cudaSuccess) {
-      set_error("cudaStreamWaitEvent failed while forking segment %d", i + 1);
+      set_error("cudaStreamWaitEvent failed while forking line %d", i + 1);
       rc = SP_ERR_CUDA;
       break;
     }
     forked = i + 1;
-    if (rc == SP_OK) rc = launch_segment(segs[i + 1], slots, items, jobs, tw, P->streams[i]);
+    if (rc == SP_OK) rc = launch_line(lines[i + 1], slots, items, jobs, tw, true, P->streams[i]);
   }
-  if (rc == SP_OK) rc = launch_segment(segs[0], slots, items, jobs, tw, st);
+  if (rc == SP_OK) rc = launch_line(lines[0], slots, items, jobs, tw, n_aux > 0, st);
   for (int i = 0; i < forked; ++i) {
     const cudaError_t e1 = cudaEventRecord(P->events[1 + i], P->streams[i]);
     const cudaError_t e2 = cudaStreamWaitEvent(st, P->events[1 + i], 0);
     if (rc == SP_OK && (e1 != cudaSuccess || e2 != cudaSuccess)) {
-      set_error("joining segment %d failed: %s", i + 1,
-                cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
+      set_error("joining line %d failed: %s", i + 1, cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
       rc = SP_ERR_CUDA;
     }
   }
@@ -443,7 +475,7 @@ extern "C" int sp_engine_workspace_size(const sp_trial* trials, int n_trials, si
   return SP_OK;
 }
 
-// sp_engine_run's body; `concurrent` lets the chains of different sizes run
+// sp_engine_run's body; `concurrent` lets the lines of different sizes run
 // on forked auxiliary streams (sp_engine_run_static keeps them on `stream`:
 // it creates no streams or events).
 int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, size_t workspace_bytes,
@@ -502,7 +534,9 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       if (count == 0) continue;
       int occ[kPassKinds], sms = 1;
       SP_CUDA_TRY(occupancy_for(N, E, occ, &sms));
-      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, sms, 0};
+      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, sms, 1.0, 0.0, 0};
+      for (int i = gstart[g]; i < gstart[g + 1]; ++i)
+        if (trials[i].n == N) sg.work += (double)N * N * (uses_dm(trials[i]) ? 2 : 1);
       for (int i = gstart[g]; i < gstart[g + 1]; ++i)
         if (trials[i].n == N) sg.ticks = std::max(sg.ticks, trials[i].n_iter + 1);
       // Partially coherent slots project in their own kernels: the column
@@ -519,6 +553,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
         if (opts && opts->ctas_per_sm > 0) per_sm = std::min(per_sm, (int)opts->ctas_per_sm);
         const int units = count * pass_units(N, E, sg.kind[p]);
         sg.grid[p] = std::max(1, std::min(units, sms * per_sm));
+        sg.rounds = (double)units / (sms * per_sm);  // (of the row pass, the last)
       }
       for (int i = gstart[g]; i < gstart[g + 1]; ++i) {
         if (trials[i].n != N || !partial(trials[i])) continue;
@@ -614,16 +649,16 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
   const int2* djobs = reinterpret_cast<const int2*>(ws + L.jobs_off);
   const bool use_graph = opts && opts->use_graph && st != nullptr;
   g_last_launches = (int64_t)L.mt_first.size();
-  size_t max_segs = 1;
   for (int g = 0; g < n_groups; ++g) {
-    max_segs = std::max(max_segs, segs[g].size());
     for (const Segment& sg : segs[g]) {
       g_last_launches += sg.ticks + std::min(sg.ticks, sg.col_ticks);
       g_last_launches += (int64_t)__builtin_popcount(sg.pc_mask) * sg.ticks;
     }
   }
-  // auxiliary streams for concurrent segment chains, made before any capture
+  // auxiliary streams for concurrent lines, made before any capture
   ForkPool* pool = nullptr;
+  size_t max_segs = 1;
+  for (const auto& v : segs) max_segs = std::max(max_segs, v.size());
   if (concurrent && max_segs > 1) SP_CUDA_TRY(fork_pool(dev, (int)max_segs - 1, &pool));
 
   for (int g = 0; g < n_groups; ++g) {

@@ -14,9 +14,48 @@ struct PassArgs {
   int tick_off;
   const float2* tw;
   int reverse;  // walk the item list from its end
+  int overlap;  // independent of the previous kernel of the stream (see chain_start)
+  int late;     // let the next kernel in only at the last item
 };
 
-
+// The waits of programmatic launches (see pdl_allow_next).  A kernel whose
+// planes are the previous kernel's output waits for it before its first item;
+// one that only needs earlier kernels (another size's pass ran in between)
+// starts at once, on the SMs that the previous kernel's last round leaves idle,
+// and waits after its first item.  Either way it lets the next kernel in only
+// after its wait, so when a kernel starts everything before its predecessor is
+// complete.  With `late`, each CTA lets it in only when it begins its last item:
+// CTAs let in earlier hold SMs that a concurrent line of launches could use (20 x
+// 512^2 beside 12 x 256^2: 86 against 91 us per iteration; alone, earlier is better,
+// 4 x 2048^2 266 against 268).
+// LINE kernels know both flags; the others, for a size alone on the chip, wait
+// and let go at their start (the flags' code in the loop costs the 2048^2 passes
+// 2%).
+template <bool LINE>
+__device__ __forceinline__ void chain_start(const PassArgs& a) {
+  if (LINE && a.overlap) return;
+  pdl_wait_prev();
+  if (!(LINE && a.late)) pdl_allow_next();
+}
+template <bool LINE>
+__device__ __forceinline__ void chain_top(const PassArgs& a, int k, bool last) {  // before item k
+  if constexpr (LINE) {
+    if (a.overlap && k == 1) {
+      pdl_wait_prev();
+      if (!a.late) pdl_allow_next();
+    }
+    if (a.late && last && (k > 0 || !a.overlap)) pdl_allow_next();
+  }
+}
+template <bool LINE>
+__device__ __forceinline__ void chain_end(const PassArgs& a, bool one_item) {
+  if constexpr (LINE) {
+    if (a.overlap && one_item) {
+      pdl_wait_prev();
+      pdl_allow_next();
+    }
+  }
+}
 
 // Copy one slot descriptor into shared memory (word by word).
 __device__ __forceinline__ void load_slot(Slot* dst, const Slot* __restrict__ src) {
@@ -82,7 +121,7 @@ __device__ __forceinline__ const float2* stage_twiddles(float2* tw, const float2
 // requested as soon as its psi rows of the current item have been consumed,
 // together with the descriptor of the item after that; the item list is read
 // ahead into registers.
-template <int N, int E, int TH>
+template <int N, int E, int TH, bool LINE>
 __global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
     row_pass_kernel(PassArgs a) {
   using SM = RowSmem<N, E, TH>;
@@ -104,8 +143,7 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
   load_slot_by<RG::GT>(&sl[0][g], &a.slots[i0.slot], gtid);
   if (i1.slot >= 0) load_slot_by<RG::GT>(&sl[1][g], &a.slots[i1.slot], gtid);
   sync();
-  pdl_wait_prev();  // the planes are the previous pass's output
-  pdl_allow_next();
+  chain_start<LINE>(a);  // the planes are the previous pass's output
   bool ready = false;
   if (row_finishes(sl[0][g], tick)) {
     prefetch_row_tile<N, E, TH>(sl[0][g], i0.block, smem, g, gtid);
@@ -113,8 +151,10 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
     ready = true;
   }
   int par = 0;
+  const bool one_item = it + G >= n_sub;
   for (int k = 0; it < n_sub; it += G, ++k) {
     const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
+    chain_top<LINE>(a, k, it + G >= n_sub);
     sync();  // the group is done with its rows of both buffers and with item k-1's slot entry
     const Slot& s = sl[k % 3][g];
     auto copy_ring = [&]() {  // item k+2's descriptor into item k-1's entry
@@ -142,6 +182,7 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
     i1 = i2;
     i2 = i3;
   }
+  chain_end<LINE>(a, one_item);
   cp_async_wait_all();
 }
 
@@ -155,7 +196,7 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, true) * (kThreads / TH))
 // round a ring of three (items k, k+1 and k+2, whose copy is requested during
 // item k), and the item list is read ahead into registers, so no step of the
 // loop waits on a global load.
-template <int N, int E, int TH>
+template <int N, int E, int TH, bool LINE>
 __global__ void __launch_bounds__(TH, min_blocks_for(E, false) * (kThreads / TH))
     col_pass_kernel(PassArgs a) {
   using CS = ColSmem<N, E, TH>;
@@ -174,15 +215,16 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, false) * (kThreads / TH)
   load_slot(&sl[0], &a.slots[i0.slot]);
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
-  pdl_wait_prev();  // the planes (and the transposed modulus) are earlier kernels' output
-  pdl_allow_next();
+  chain_start<LINE>(a);  // the planes (and the transposed modulus) are earlier kernels' output
   copy_col_g<N, E, TH>(sl[0], i0.block, tick, smem);
   asm volatile("cp.async.commit_group;" ::: "memory");
   float2* pend = nullptr;  // plane whose last stage is left in the other buffer
   int pend_block = 0;
   int b = 0;
+  const bool one_item = it + G >= n_sub;
   for (int k = 0; it < n_sub; it += G, ++k, b ^= 1) {
     const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
+    chain_top<LINE>(a, k, it + G >= n_sub);
     cp_async_wait_all();  // this item's G tile and item k+1's slot descriptor
     __syncthreads();      // ... visible to all; the previous item is finished
     float2* other = smem + (b ^ 1) * CS::kB;
@@ -207,6 +249,7 @@ __global__ void __launch_bounds__(TH, min_blocks_for(E, false) * (kThreads / TH)
     i1 = i2;
     i2 = i3;
   }
+  chain_end<LINE>(a, one_item);
   __syncthreads();
   if (pend) col_last_stage<N, E, TH>(pend, pend_block, smem + (b ^ 1) * CS::kB, tw, [] {});
   cp_async_wait_all();
@@ -235,7 +278,7 @@ __host__ __device__ constexpr int col_split(int N, int E) {
   return col_single_buffered(N, E) ? pass_split(N, E, kColSbThreads) : 1;
 }
 
-template <int N, int E>
+template <int N, int E, bool LINE>
 __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs a) {
   constexpr int TH = kColSbThreads;
   constexpr int SPLIT = col_split(N, E);
@@ -256,14 +299,15 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
   load_slot(&sl[0], &a.slots[i0.slot]);
   if (i1.slot >= 0) load_slot(&sl[1], &a.slots[i1.slot]);
   __syncthreads();
-  pdl_wait_prev();  // the planes (and the transposed modulus) are earlier kernels' output
-  pdl_allow_next();
+  chain_start<LINE>(a);  // the planes (and the transposed modulus) are earlier kernels' output
   copy_col_mod<N, E, TH>(sl[0], i0.block, tick, mod);
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (col_projects(sl[0], tick)) copy_col_tile<N, E, TH>(sl[0].g, i0.block, tile);
   asm volatile("cp.async.commit_group;" ::: "memory");
+  const bool one_item = it + G >= n_sub;
   for (int k = 0; it < n_sub; it += G, ++k) {
     const Item i3 = sub_item<SPLIT>(a, it + 3 * G);
+    chain_top<LINE>(a, k, it + G >= n_sub);
     cp_async_wait_all();  // this sub-item's modulus and tile, sub-item k+1's descriptor
     __syncthreads();      // ... visible to all; the previous sub-item is finished
     const Slot& s = sl[k % 3];
@@ -287,6 +331,7 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
     i1 = i2;
     i2 = i3;
   }
+  chain_end<LINE>(a, one_item);
   cp_async_wait_all();
 }
 
@@ -306,8 +351,17 @@ __host__ __device__ constexpr bool has_small_ctas(int N, int E) {
   return N >= 64 && N <= 512 && pass_split(N, E, kSmallThreads) > 1;
 }
 
-// pass kinds: 0 column, 1 row, and the same in small CTAs
-enum { kPassCol = 0, kPassRow = 1, kPassColSmall = 2, kPassRowSmall = 3, kPassKinds = 4 };
+// pass kinds: 0 column, 1 row, the same in small CTAs, and the same (large) for
+// lines of several sizes
+enum {
+  kPassCol = 0,
+  kPassRow = 1,
+  kPassColSmall = 2,
+  kPassRowSmall = 3,
+  kPassColLine = 4,
+  kPassRowLine = 5,
+  kPassKinds = 6
+};
 
 template <int N, int E, int TH>
 constexpr size_t col_smem_bytes() {
@@ -323,20 +377,24 @@ constexpr size_t row_smem_bytes() { return (size_t)RowSmem<N, E, TH>::kTotal * s
 // cudaErrorInvalidValue for one that is not compiled.
 template <int N, int E, class F>
 cudaError_t with_pass_kernel(int which, F&& f) {
-  if (which == kPassCol) {
+  auto large = [&](auto line, bool col) {
+    constexpr bool LINE = decltype(line)::value;
+    if (!col)
+      return f(row_pass_kernel<N, E, kThreads, LINE>, kThreads, row_smem_bytes<N, E, kThreads>());
     if constexpr (col_single_buffered(N, E))
-      return f(col_pass_sb_kernel<N, E>, kColSbThreads, col_smem_bytes<N, E, kColSbThreads>());
+      return f(col_pass_sb_kernel<N, E, LINE>, kColSbThreads, col_smem_bytes<N, E, kColSbThreads>());
     else
-      return f(col_pass_kernel<N, E, kThreads>, kThreads, col_smem_bytes<N, E, kThreads>());
-  }
-  if (which == kPassRow)
-    return f(row_pass_kernel<N, E, kThreads>, kThreads, row_smem_bytes<N, E, kThreads>());
+      return f(col_pass_kernel<N, E, kThreads, LINE>, kThreads, col_smem_bytes<N, E, kThreads>());
+  };
+  if (which == kPassCol || which == kPassRow) return large(std::false_type{}, which == kPassCol);
+  if (which == kPassColLine || which == kPassRowLine)
+    return large(std::true_type{}, which == kPassColLine);
   if constexpr (has_small_ctas(N, E)) {
     if (which == kPassColSmall)
-      return f(col_pass_kernel<N, E, kSmallThreads>, kSmallThreads,
+      return f(col_pass_kernel<N, E, kSmallThreads, false>, kSmallThreads,
                col_smem_bytes<N, E, kSmallThreads>());
     if (which == kPassRowSmall)
-      return f(row_pass_kernel<N, E, kSmallThreads>, kSmallThreads,
+      return f(row_pass_kernel<N, E, kSmallThreads, false>, kSmallThreads,
                row_smem_bytes<N, E, kSmallThreads>());
   }
   return cudaErrorInvalidValue;
@@ -354,7 +412,7 @@ template <int N, int E>
 cudaError_t pass_setup_t(int* occupancy) {
   for (int which = 0; which < kPassKinds; ++which) {
     occupancy[which] = 0;
-    if (which >= kPassColSmall && !has_small_ctas(N, E)) continue;
+    if ((which == kPassColSmall || which == kPassRowSmall) && !has_small_ctas(N, E)) continue;
     const cudaError_t e =
         with_pass_kernel<N, E>(which, [&](void (*k)(PassArgs), int threads, size_t smem) {
           cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -374,8 +432,8 @@ inline bool use_small_ctas(int N, int E, int items, int sms) {
 
 // work units of one item in each pass kind
 inline int pass_units(int N, int E, int which) {
-  if (which == kPassCol) return col_split(N, E);
-  if (which == kPassRow) return 1;
+  if (which == kPassCol || which == kPassColLine) return col_split(N, E);
+  if (which == kPassRow || which == kPassRowLine) return 1;
   return pass_split(N, E, kSmallThreads);
 }
 

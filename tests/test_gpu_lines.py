@@ -1,0 +1,67 @@
+"""Batches whose sizes fill the chip run in one line of overlapping launches,
+the others beside it: every trial equals itself alone, bit for bit, whatever it
+shares the call with, for different iteration counts and algorithms, eager, as
+a graph, and with a partially coherent size in the line."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mix", [
+    # (N, trials, iterations, algorithm), sizes in more than one round of SMs among them
+    ((512, 10, 5, "hio"), (1024, 3, 7, "raar")),
+    ((256, 40, 4, "dm"), (512, 9, 6, "hio"), (1024, 2, 3, "dm"), (2048, 1, 5, "er")),
+    ((128, 2, 9, "hio"), (512, 1, 4, "raar"), (2048, 1, 3, "hio")),
+    ((256, 38, 6, "er"), (512, 9, 4, "ipsf"), (1024, 2, 5, "hio"))])
+def test_mixed_lines_match_alone(mix):
+    import torch
+    from als_speckle_b200.engine import Engine, TrialSpec
+    from als_speckle_b200.workloads import gaussian_ipsf
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    pat = {}
+    for N, _, _, _ in mix:
+        S = torch.zeros((N, N), device="cuda")
+        S[N // 8:N // 2, N // 4:N // 2 + 3] = 1
+        pat[N] = (30 * torch.rand((N, N), generator=g, device="cuda"), S)
+
+    def specs(sel):
+        out, k = [], 0
+        for N, count, its, alg in mix:
+            for _ in range(count):
+                if sel is None or k in sel:
+                    ip = torch.from_numpy(gaussian_ipsf(N, 1.5)).cuda() if alg == "ipsf" else None
+                    out.append(TrialSpec(
+                        psi=torch.zeros((N, N), dtype=torch.complex64, device="cuda"), modulus=pat[N][0],
+                        support=pat[N][1], iterations=its, order=((alg if ip is None else "hio", its),),
+                        beta=0.9, random_phase=True, seed=2, trial=k, ipsf=ip))
+                k += 1
+        return out, k
+
+    _, total = specs(set())
+    stream = torch.cuda.Stream()
+    batches = []
+    for use_graph in (False, True):
+        eng = Engine(use_graph=use_graph)
+        sp, _ = specs(None)
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for _ in range(3):  # back to back: a round of launches right behind the last one's
+                eng.solve(sp, stream=stream)
+        stream.synchronize()
+        batches.append([s.psi.cpu().numpy() for s in sp])
+        eng.close()
+    ends = np.cumsum([m[1] for m in mix])
+    picks = sorted({0, total - 1} | {int(e) - 1 for e in ends} | {int(e) for e in ends[:-1]})
+    eng = Engine(use_graph=False)
+    for k in picks:
+        sp, _ = specs({k})
+        eng.solve(sp)
+        torch.cuda.synchronize()
+        alone = sp[0].psi.cpu().numpy()
+        for b in batches:
+            np.testing.assert_array_equal(b[k], alone)
+    for a, b in zip(*batches):
+        np.testing.assert_array_equal(a, b)
+    eng.close()
