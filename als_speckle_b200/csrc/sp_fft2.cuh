@@ -345,7 +345,8 @@ struct PhasorSum {
 // 1/sqrt(1 + (g - |F|)^2 / g^2) summed (phasing_rftf_accumulate.cl), g the goal
 // modulus.  1/sqrt(x) by the reciprocal square root and one Newton step;
 // nothing needs a slow form (at g = 0 the quotient is infinite, or NaN for
-// F = 0 too, as in the division).
+// F = 0 too, as in the division; a square past the range leaves |F| infinite
+// and the summand 0, as a square root would).
 struct RftfSum {
   const float* goal;
   struct Pixel {
@@ -359,7 +360,8 @@ struct RftfSum {
     return {g, 1.f / (g * g)};
   }
   __device__ __forceinline__ bool add(float& acc, float2 v, Pixel p) const {
-    const float d1 = p.g - sqrtf(v.x * v.x + v.y * v.y);
+    const float p2 = v.x * v.x + v.y * v.y;
+    const float d1 = p.g - (p2 > 0.f && p2 < 3e38f ? p2 * rsqrtf(p2) : p2);
     const float x = 1.f + (d1 * d1) * p.inv;
     float r = rsqrtf(x);
     if (x < 1e30f) r = r * fmaf(-0.5f * x * r, r, 1.5f);

@@ -29,14 +29,6 @@ namespace sp {
 
 static inline int upsampled_points(int U) { return (3 * U + 1) / 2; }  // ceil(1.5 U)
 
-// exp(2 pi i num / den) with num reduced modulo den exactly first
-__device__ __forceinline__ float2 turn(long long num, long long den) {
-  long long r = num % den;
-  if (r < 0) r += den;
-  float s, c;
-  sincospif(2.0f * (float)((double)r / (double)den), &s, &c);
-  return make_float2(c, s);
-}
 // the signed coarse shift d0 of frame f from its argmax key
 __device__ __forceinline__ int2 coarse_shift(unsigned long long key, int N) {
   const uint32_t sidx = 0xffffffffu - (uint32_t)(key & 0xffffffffu);

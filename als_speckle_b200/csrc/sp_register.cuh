@@ -139,48 +139,44 @@ struct RegPeakOp {
   }
 };
 
+// exp(2 pi i num / den) with num reduced modulo den exactly first
+__device__ __forceinline__ float2 turn(long long num, long long den) {
+  long long r = num % den;
+  if (r < 0) r += den;
+  float s, c;
+  sincospif(2.0f * (float)((double)r / (double)den), &s, &c);
+  return make_float2(c, s);
+}
+
 // Rows of F exp(2 pi i k.d/N) exp(-i theta), d = num / U, inverse, transposed
-// into X.  With num = d0 U + (p - h) per axis the ramp factors into the
-// whole-pixel turn exp(2 pi i k d0 / N) and the kernel-table entry
-// W[k][p] = exp(2 pi i k (p - h)/(U N)); the plane's column factors are
-// gathered once per plane, and the turns come from a table of the CTA (with
-// a sincospi and the shift's divisions at every element, and FP64 sin and cos
-// of theta, the elementwise pass alone took 106 us for 128 planes of 256^2).
+// into X.  The ramp is a row factor exp(2 pi i ky dy/N - i theta) times a column
+// factor exp(2 pi i kx dx/N), made once per line and once per plane, so an
+// element takes two products (106 us for 128 planes of 256^2 as an elementwise
+// pass with a sincospi, the shift's divisions and FP64 sin and cos of theta at
+// every element, 64 us with the ramp composed of table entries in this kernel,
+// now 29 us with the transform).
 struct RegShiftOp {
   RegArgs a;
   int planes, lines;
-  static constexpr int extra(int N) { return 2 * N; }  // column factors | exp(2 pi i r/N)
-  // floor division of a numerator by U: d = d0 U + (p - h), p - h in [-h, h]
-  __device__ __forceinline__ int whole(int d) const {
-    const int e = d + a.M / 2;
-    return e >= 0 ? e / a.U : -((-e + a.U - 1) / a.U);
-  }
-  __device__ void init(float2* ex) const {
-    for (int r = threadIdx.x; r < lines; r += kThreads) ex[lines + r] = turn_pow2(r, lines);
-  }
+  static constexpr int extra(int N) { return N; }  // column factors
+  __device__ void init(float2*) const {}
   __device__ void prepare(int f, float2* ex) const {
     __syncthreads();  // the previous plane's loads are done
-    const int dx = a.num[f].y;
-    const int px = dx - whole(dx) * a.U + a.M / 2;
-    for (int k = threadIdx.x; k < lines; k += kThreads) ex[k] = a.W[(size_t)k * a.M + px];
+    const int nx = a.num[f].y;
+    for (int k = threadIdx.x; k < lines; k += kThreads)
+      ex[k] = turn((long long)signed_freq(k, lines) * nx, (long long)a.U * lines);
     __syncthreads();
   }
   struct Line {
     const float2* F;
-    float2 wy, cs;
-    int ty, d0x;
+    float2 w;
   };
   __device__ __forceinline__ Line line(int f, int ky) const {
-    const int2 d = a.num[f];
-    const int d0y = whole(d.x);
-    const int py = d.x - d0y * a.U + a.M / 2;
-    return {a.F + ((size_t)f * lines + ky) * lines, a.W[(size_t)ky * a.M + py], a.cs[f],
-            signed_freq(ky, lines) * d0y, whole(d.y)};
+    return {a.F + ((size_t)f * lines + ky) * lines,
+            cmul(turn((long long)signed_freq(ky, lines) * a.num[f].x, (long long)a.U * lines), a.cs[f])};
   }
   __device__ __forceinline__ float2 load(const Line& l, int kx, const float2* ex) const {
-    float2 w = ex[lines + ((l.ty + signed_freq(kx, lines) * l.d0x) & (lines - 1))];
-    w = cmul(w, cmul(l.wy, ex[kx]));
-    return cmul(l.F[kx], cmul(w, l.cs));
+    return cmul(l.F[kx], cmul(l.w, ex[kx]));
   }
   template <int N, class Sync>
   __device__ __forceinline__ void done(int f, int l0, int nl, const float2 (&v)[Lines<N>::E],

@@ -60,3 +60,16 @@ def test_rftf_of_embedded_frames(N, frames, rows, cols):
             want += 1 / np.sqrt(1 + (g.astype(np.float64) - F) ** 2 / g.astype(np.float64) ** 2)
     got = gpu_rftf(None, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()).cpu().numpy()
     assert np.max(np.abs(got - np.fft.fftshift(want / frames))) < 2e-5
+
+
+def test_rftf_of_extreme_magnitudes():
+    """Transforms whose squares leave the float range count as the summand's
+    limits: 0 where |F|^2 overflows, g-only where |F| = 0."""
+    import torch
+    from als_speckle_b200.phasing import gpu_rftf
+    x = np.zeros((2, 4, 4), np.complex64)
+    x[0, 0, 0] = 3e19  # |F|^2 = inf everywhere
+    g = np.ones((16, 16), np.float32)
+    got = gpu_rftf(None, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()).cpu().numpy()
+    # frame 1: F = 0, summand 1/sqrt(2)
+    assert np.allclose(got, 0.5 / np.sqrt(2.0), rtol=1e-6)
