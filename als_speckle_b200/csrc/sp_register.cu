@@ -59,10 +59,14 @@ __global__ void reg_kernel_table(float2* __restrict__ W, int N, int U, int M) {
 // a row pair from shared memory, and a lane the columns lane + 32 m, m < MQ.
 // Shared memory is the next limit (pairing re with im instead needs twice the A
 // loads and ran at its bandwidth: 245 us), so a warp keeps R as large as the
-// registers allow; four 128-thread CTAs per SM cover one another's staging.
-// 128 frames, N = 256, M = 96: rows 178 us (FMA pipes 62% busy) and columns
-// 69 us; 557 and 234 us with scalar FMAs on 4 x 3 and 1 x 3 tiles.
-constexpr int kRegK = 32, kRegThreads = 128, kRegWarps = kRegThreads / 32;
+// registers allow; four 128-thread CTAs per SM.  Staged one chunk ahead of the
+// products, since four CTAs alone did not cover the loads.
+// 128 frames, N = 256, M = 96: rows 154 us (178 staged between two barriers,
+// FMA pipes 62% busy; 557 with scalar FMAs on 4 x 3 tiles), columns 70 us (the
+// loads of A are few there: 69, 234).  The whole call at U = 10, 42, 64, 85,
+// 100, 170: 210, 266, 342, 441, 546, 919 us; staged between barriers 254, 302,
+// 365, 450, 550, 914.
+constexpr int kRegK = 16, kRegThreads = 128, kRegWarps = kRegThreads / 32;
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 r;
@@ -79,36 +83,59 @@ __host__ __device__ constexpr int reg_pairs(int MQ) { return MQ <= 4 ? 4 : 2; }
 __host__ __device__ constexpr int reg_tile_rows(int MQ) { return kRegWarps * 2 * reg_pairs(MQ); }
 
 // re[j][m], im[j][m]: the two rows of the warp's pair j, column lane + 32 m.
-// `as` holds [pair of the tile][k], `bs` [k][M].
+// `as` holds [pair of the tile][k], `bs` [k][M], two chunks of kRegK each: while
+// one is multiplied the next one's B is copied and its A values travel through
+// the threads' registers (Src::fetch, then Src::make).  Thread i always stages
+// position i % kRegK of the chunk, of pairs i / kRegK + 8 u.
 template <int MQ, class Src>
 __device__ __forceinline__ void reg_product(float2 (&re)[reg_pairs(MQ)][MQ],
                                             float2 (&im)[reg_pairs(MQ)][MQ], const Src& src, int K, int M,
                                             float4* as, float2* bs) {
-  constexpr int R = reg_pairs(MQ);
+  constexpr int R = reg_pairs(MQ), PAIRS = kRegWarps * R, STEP = kRegThreads / kRegK;
+  constexpr int U = PAIRS / STEP;
+  static_assert(U * STEP == PAIRS, "whole pairs per thread");
   const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int kt = threadIdx.x % kRegK, pt = threadIdx.x / kRegK;
 #pragma unroll
   for (int j = 0; j < R; ++j)
 #pragma unroll
     for (int m = 0; m < MQ; ++m) re[j][m] = im[j][m] = make_float2(0.f, 0.f);
-  for (int k0 = 0; k0 < K; k0 += kRegK) {
-    const int nk = K - k0 < kRegK ? K - k0 : kRegK;  // K = N: 8 and 16 are shorter
-    __syncthreads();  // the previous chunk's tiles are consumed
-    // nk rows of B are contiguous; nk and k0 are multiples of 8, so they are
-    // whole 16-byte pieces
+  typename Src::Raw raw[U];
+  auto fetch = [&](int k0) {
+    // rows of B are contiguous; k0 and the chunk's length are multiples of 8, so
+    // they are whole 16-byte pieces
+    const int nk = K - k0 < kRegK ? K - k0 : kRegK;
+    float2* dst = bs + (k0 / kRegK % 2) * kRegK * M;
     for (int i = threadIdx.x; i < nk * M / 2; i += kRegThreads)
-      cp_async<16>(bs + 2 * i, src.b + (size_t)k0 * M + 2 * i);
-    src.stage(k0, nk, as, kRegWarps * R);
+      cp_async<16>(dst + 2 * i, src.b + (size_t)k0 * M + 2 * i);
+    if (kt < nk) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) raw[u] = src.fetch(pt + u * STEP, k0 + kt);
+    }
+  };
+  auto put = [&](int k0) {
+    if (k0 + kt < K) src.make(raw, as + (k0 / kRegK % 2) * PAIRS * kRegK + kt, pt, k0 + kt);
     cp_async_wait_all();
     __syncthreads();
-#pragma unroll 4
+  };
+  __syncthreads();  // (what the source prepared)
+  fetch(0);
+  put(0);
+  for (int k0 = 0; k0 < K; k0 += kRegK) {
+    const bool more = k0 + kRegK < K;
+    if (more) fetch(k0 + kRegK);
+    const int nk = K - k0 < kRegK ? K - k0 : kRegK;
+    const float4* ac = as + (k0 / kRegK % 2) * PAIRS * kRegK;
+    const float2* bc = bs + (k0 / kRegK % 2) * kRegK * M;
+#pragma unroll(MQ == 4 ? 2 : 4)  // (MQ = 4 spills at 4; the wider ones, with half the pairs, don't)
     for (int kk = 0; kk < nk; ++kk) {
       float4 a[R];
 #pragma unroll
-      for (int j = 0; j < R; ++j) a[j] = as[(w * R + j) * kRegK + kk];
+      for (int j = 0; j < R; ++j) a[j] = ac[(w * R + j) * kRegK + kk];
 #pragma unroll
       for (int m = 0; m < MQ; ++m) {
         const int q = lane + 32 * m;
-        const float2 b = bs[kk * M + (q < M ? q : 0)];
+        const float2 b = bc[kk * M + (q < M ? q : 0)];
         const float2 bx = make_float2(b.x, b.x), by = make_float2(b.y, b.y);
         const float2 ny = make_float2(-b.y, -b.y);
 #pragma unroll
@@ -119,31 +146,44 @@ __device__ __forceinline__ void reg_product(float2 (&re)[reg_pairs(MQ)][MQ],
         }
       }
     }
+    if (more) put(k0 + kRegK);  // (the other half: its last readers passed the barrier before)
   }
 }
 
+// The modulation's products with their contraction spelled out: left to the
+// compiler it depends on the code around them, and frames whose two best grid
+// points agree to the last bits then move to the other one.
+__device__ __forceinline__ float2 reg_cmul(float2 a, float2 w) {
+  return make_float2(fmaf(a.x, w.x, -__fmul_rn(a.y, w.y)), fmaf(a.x, w.y, __fmul_rn(a.y, w.x)));
+}
+__device__ __forceinline__ float2 reg_cmulc(float2 a, float2 w) {  // a conj(w)
+  return make_float2(fmaf(a.x, w.x, __fmul_rn(a.y, w.y)), fmaf(a.y, w.x, -__fmul_rn(a.x, w.y)));
+}
+
 // A = X_f' of one frame's rows ky0 ..: the modulation is separable, the row
-// factors exp(2 pi i ky d0y/N) made once, a chunk's column factors once each.
+// factors exp(2 pi i ky d0y/N) made once, the column factors once per position.
 struct RegRowsSrc {
   const float2 *F, *R, *b;
-  float2 *rowf, *colf;
-  int N, ky0;
-  int2 d0;
-  __device__ __forceinline__ float2 at(int rr, int k) const {
-    if (ky0 + rr >= N) return make_float2(0.f, 0.f);
-    const size_t idx = (size_t)(ky0 + rr) * N + k;
-    return cmul(cmul(cmulc(F[idx], R[idx]), rowf[rr]), colf[k % kRegK]);
+  const float2* rowf;
+  int N, ky0, d0x;
+  struct Raw {
+    float2 f0, r0, f1, r1;
+  };
+  __device__ __forceinline__ Raw fetch(int p, int k) const {
+    const float2 z = make_float2(0.f, 0.f);
+    if (ky0 + 2 * p >= N) return {z, z, z, z};  // (N is even)
+    const size_t idx = (size_t)(ky0 + 2 * p) * N + k;
+    return {F[idx], R[idx], F[idx + N], R[idx + N]};
   }
-  __device__ void stage(int k0, int nk, float4* as, int pairs) const {
-    if (threadIdx.x < nk) colf[threadIdx.x] = turn_pow2(signed_freq(k0 + threadIdx.x, N) * d0.y, N);
-    __syncthreads();
-#pragma unroll 4
-    for (int i = threadIdx.x; i < pairs * kRegK; i += kRegThreads) {
-      const int p = i / kRegK, kk = i % kRegK;
-      if (kk < nk) {
-        const float2 u = at(2 * p, k0 + kk), v = at(2 * p + 1, k0 + kk);
-        as[i] = make_float4(u.x, v.x, u.y, v.y);
-      }
+  template <int U>
+  __device__ __forceinline__ void make(const Raw (&raw)[U], float4* as, int pt, int k) const {
+    const float2 col = turn_pow2(signed_freq(k, N) * d0x, N);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int p = pt + u * (kRegThreads / kRegK);
+      const float2 x = reg_cmul(reg_cmul(reg_cmulc(raw[u].f0, raw[u].r0), rowf[2 * p]), col);
+      const float2 y = reg_cmul(reg_cmul(reg_cmulc(raw[u].f1, raw[u].r1), rowf[2 * p + 1]), col);
+      as[p * kRegK] = make_float4(x.x, y.x, x.y, y.y);
     }
   }
 };
@@ -154,14 +194,14 @@ __global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_rows_kernel(
     const unsigned long long* __restrict__ best, float2* __restrict__ T1, int N, int M) {
   constexpr int R = reg_pairs(MQ), ROWS = reg_tile_rows(MQ);
   extern __shared__ float4 reg_sm[];
-  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS / 2 * kRegK);
-  __shared__ float2 rowf[ROWS], colf[kRegK];
+  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS * kRegK);
+  __shared__ float2 rowf[ROWS];
   const int f = blockIdx.y, ky0 = blockIdx.x * ROWS;
   const int2 d0 = coarse_shift(best[f], N);
   for (int r = threadIdx.x; r < ROWS; r += kRegThreads)
     rowf[r] = turn_pow2(signed_freq(ky0 + r, N) * d0.x, N);
   float2 re[R][MQ], im[R][MQ];
-  const RegRowsSrc src{F + (size_t)f * N * N, Rf, W, rowf, colf, N, ky0, d0};
+  const RegRowsSrc src{F + (size_t)f * N * N, Rf, W, rowf, N, ky0, d0.y};
   reg_product<MQ>(re, im, src, N, M, reg_sm, bs);
 #pragma unroll
   for (int j = 0; j < R; ++j) {
@@ -181,14 +221,20 @@ __global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_rows_kernel(
 struct RegColsSrc {
   const float2 *W, *b;
   int M, p0;
-  __device__ void stage(int k0, int nk, float4* as, int pairs) const {
+  struct Raw {
+    float2 w0, w1;
+  };
+  __device__ __forceinline__ Raw fetch(int p, int k) const {
     const float2 zero = make_float2(0.f, 0.f);
-    for (int i = threadIdx.x; i < pairs * nk; i += kRegThreads) {
-      const int p = i % pairs, kk = i / pairs;  // neighbouring threads: neighbouring p
-      const float2* w = W + (size_t)(k0 + kk) * M + p0 + 2 * p;
-      const float2 u = p0 + 2 * p < M ? w[0] : zero, v = p0 + 2 * p + 1 < M ? w[1] : zero;
-      as[p * kRegK + kk] = make_float4(u.x, v.x, u.y, v.y);
-    }
+    const float2* w = W + (size_t)k * M + p0 + 2 * p;
+    return {p0 + 2 * p < M ? w[0] : zero, p0 + 2 * p + 1 < M ? w[1] : zero};
+  }
+  template <int U>
+  __device__ __forceinline__ void make(const Raw (&raw)[U], float4* as, int pt, int) const {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      as[(pt + u * (kRegThreads / kRegK)) * kRegK] =
+          make_float4(raw[u].w0.x, raw[u].w1.x, raw[u].w0.y, raw[u].w1.y);
   }
 };
 
@@ -198,7 +244,7 @@ __global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_cols_kernel(
     unsigned long long* __restrict__ best_up) {
   constexpr int R = reg_pairs(MQ), ROWS = reg_tile_rows(MQ);
   extern __shared__ float4 reg_sm[];
-  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS / 2 * kRegK);
+  float2* bs = reinterpret_cast<float2*>(reg_sm + ROWS * kRegK);
   const int f = blockIdx.y, p0 = blockIdx.x * ROWS;
   float2 re[R][MQ], im[R][MQ];
   const RegColsSrc src{W, T1 + (size_t)f * N * M, M, p0};
@@ -232,7 +278,7 @@ __global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_cols_kernel(
 template <int MQ>
 static cudaError_t reg_upsample(const RegArgs& a, int N, unsigned long long* best_up, cudaStream_t st) {
   constexpr int rows = reg_tile_rows(MQ);
-  const int smem = (int)(sizeof(float4) * rows / 2 * kRegK + sizeof(float2) * (size_t)kRegK * a.M);
+  const int smem = (int)(sizeof(float4) * rows * kRegK + sizeof(float2) * 2 * (size_t)kRegK * a.M);
   cudaError_t e = cudaFuncSetAttribute(reg_upsample_rows_kernel<MQ>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
