@@ -179,16 +179,16 @@ __global__ void prtf_accumulate_kernel(int frames, const float2* __restrict__ ff
 }
 
 // acc += the phasor sums
-__global__ void __launch_bounds__(256) phasor_sum_kernel(const float2* __restrict__ part, SumsAt at,
-                                                         float2* __restrict__ acc, int N) {
+__global__ void __launch_bounds__(kFrameSumsThreads) phasor_sum_kernel(
+    const float2* __restrict__ part, SumsAt at, float2* __restrict__ acc, int N) {
   transposed_sums(part, at, N, [&](int r, int c, float2 s) {
     float2* p = acc + (int64_t)r * N + c;
     *p = make_float2(p->x + s.x, p->y + s.y);
   });
 }
 // prtf = fftshift(|phasor sums| / frames)
-__global__ void __launch_bounds__(256) prtf_sums_kernel(const float2* __restrict__ part, SumsAt at,
-                                                        float* __restrict__ prtf, int N) {
+__global__ void __launch_bounds__(kFrameSumsThreads) prtf_sums_kernel(
+    const float2* __restrict__ part, SumsAt at, float* __restrict__ prtf, int N) {
   transposed_sums(part, at, N, [&](int r, int c, float2 s) {
     prtf[(int64_t)((r + N / 2) % N) * N + (c + N / 2) % N] = hypotf(s.x / at.frames, s.y / at.frames);
   });
@@ -502,7 +502,7 @@ int sp_prtf(const void* frames, int n_frames, int rows, int cols, int N, void* w
   SumsAt at{n_frames, 1, 1};
   SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, nullptr,
                                   &at.run, &at.group_cols, st));
-  prtf_sums_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>(
+  prtf_sums_kernel<<<frame_sums_grid(N), kFrameSumsThreads, 0, st>>>(
       (const float2*)work, at, prtf, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
@@ -518,7 +518,7 @@ int sp_prtf_phasors(const void* frames, int n_frames, int rows, int cols, int N,
   SumsAt at{n_frames, 1, 1};
   SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, nullptr,
                                   &at.run, &at.group_cols, st));
-  phasor_sum_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>(
+  phasor_sum_kernel<<<frame_sums_grid(N), kFrameSumsThreads, 0, st>>>(
       (const float2*)work, at, (float2*)acc, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;

@@ -98,8 +98,8 @@ __global__ void rftf_accumulate_kernel(int frames, const float* goal, float* acc
 }
 
 // acc = fftshift(the RFTF sums / frames)
-__global__ void __launch_bounds__(256) rftf_sums_kernel(const float2* __restrict__ part, SumsAt at,
-                                                        float* __restrict__ acc, int N) {
+__global__ void __launch_bounds__(kFrameSumsThreads) rftf_sums_kernel(
+    const float2* __restrict__ part, SumsAt at, float* __restrict__ acc, int N) {
   transposed_sums(part, at, N, [&](int r, int c, float2 s) {
     acc[(int64_t)((r + N / 2) % N) * N + (c + N / 2) % N] = s.x / (float)at.frames;
   });
@@ -300,7 +300,7 @@ int sp_rftf_frames(const void* frames, int n_frames, int rows, int cols, const f
   SumsAt at{n_frames, 1, 1};
   SP_CUDA_TRY(frame_sums_dispatch(N, (const float2*)frames, (float2*)work, n_frames, rows, cols, goal,
                                   &at.run, &at.group_cols, st));
-  rftf_sums_kernel<<<frame_sums_grid(N), dim3(32, 8), 0, st>>>((const float2*)work, at, accumulation, N);
+  rftf_sums_kernel<<<frame_sums_grid(N), kFrameSumsThreads, 0, st>>>((const float2*)work, at, accumulation, N);
   SP_CUDA_TRY(cudaGetLastError());
   return SP_OK;
 }
