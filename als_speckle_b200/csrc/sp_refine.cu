@@ -376,7 +376,7 @@ int sp_refine_support(const void* avg, int rows, int cols, const double* kr, con
                       const unsigned char* mask, double local_t, double global_t, int kill_weakest,
                       void* work, size_t work_bytes, double* blurred, float* refined,
                       sp_stream_t stream) {
-  SP_CHECK(avg && kr && kc && mask && work && blurred && refined, SP_ERR_INVALID,
+  SP_CHECK(avg && work && blurred && refined && !kr == !kc && (kr || mask), SP_ERR_INVALID,
            "sp_refine_support: null pointer");
   size_t need = 0;
   const int rc = sp_refine_workspace_size(rows, cols, &need);
@@ -391,12 +391,13 @@ int sp_refine_support(const void* avg, int rows, int cols, const double* kr, con
   int* parent = reinterpret_cast<int*>(sums + total + 1);
   int* labels = parent + total;
   int* weakest = labels + total;
+  if (kr) SP_CUDA_TRY(launch_blur(avg, rows, cols, kr, kc, tmp, blurred, st));
+  if (!mask) return SP_OK;
   const dim3 grid((cols + 31) / 32, (rows + 7) / 8), block(32, 8);
   parts_init_kernel<<<grid, block, 0, st>>>(mask, parent, rows, cols);
   parts_join_kernel<<<grid, block, 0, st>>>(mask, parent, rows, cols);
   parts_label_kernel<<<grid, block, 0, st>>>(mask, parent, labels, rows, cols);
   SP_CUDA_TRY(cudaGetLastError());
-  SP_CUDA_TRY(launch_blur(avg, rows, cols, kr, kc, tmp, blurred, st));
   // (the smallest order-preserving key is 0, and so is an empty sum)
   SP_CUDA_TRY(cudaMemsetAsync(keys, 0, 16 * (size_t)(total + 1), st));
   label_stats_kernel<<<grid_of(total), 256, 0, st>>>(blurred, (const float2*)avg, labels, total, keys,

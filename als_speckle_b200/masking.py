@@ -64,7 +64,9 @@ DETECT = (0.95, 1.05)  # support values that count as inside
 def inside(data, detect_val=DETECT):
     """Mask of the (nearly binary) support's inside, as ``label_parts`` uses it."""
     data = np.asarray(data)
-    return (data >= detect_val[0]) & (data <= detect_val[1])
+    mask = data >= detect_val[0]
+    mask &= data <= detect_val[1]
+    return mask
 
 
 def label_parts(data, detect_val=DETECT):

@@ -629,7 +629,7 @@ def _gaussian_1d_kernel(n, sigma):
     ``shape.gaussian`` ``shape.py:494-508``)."""
     x = np.arange(n).astype(float)
     g = np.exp(-(x - n // 2) ** 2 / (2 * float(sigma) ** 2))
-    g = np.fft.fftshift(g)
+    g = np.concatenate((g[n - n // 2:], g[:n - n // 2]))  # fftshift
     return g / g.sum()
 
 
@@ -657,19 +657,28 @@ def refine_support(support, average_mag, blur=3, local_threshold=.2, global_thre
     if tuple(avg_t.shape) != (rows, cols):
         raise ValueError("support and average_mag must have the same shape")
     dev = avg_t.device
-    kr = torch.from_numpy(_gaussian_1d_kernel(rows, blur)).to(dev)
-    kc = kr if rows == cols else torch.from_numpy(_gaussian_1d_kernel(cols, blur)).to(dev)
-    mask = torch.from_numpy(np.ascontiguousarray(masking.inside(support)).view(np.uint8)).to(dev)
+    k = _gaussian_1d_kernel(rows, blur)
+    if rows != cols:
+        k = np.concatenate((k, _gaussian_1d_kernel(cols, blur)))
+    k = torch.from_numpy(k).to(dev)
     nbytes = C.c_size_t(0)
     call("sp_refine_workspace_size", rows, cols, C.byref(nbytes))
     work = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
-    blurred = torch.empty((rows, cols), dtype=torch.float64, device=dev)
-    refined = torch.empty((rows, cols), dtype=torch.float32, device=dev)
-    call("sp_refine_support", ptr(avg_t), rows, cols, ptr(kr), ptr(kc), ptr(mask),
-         float(local_threshold), float(global_threshold), 1 if kill_weakest else 0, ptr(work),
-         nbytes.value, ptr(blurred), ptr(refined), stream_ptr())
-    ref = refined.cpu().numpy().astype(support.dtype if support.dtype.kind == "f" else np.int64)
-    return ref, blurred.cpu().numpy()
+    out = torch.empty(12 * rows * cols, dtype=torch.uint8, device=dev)  # blurred, then refined
+    refined_ptr = out.data_ptr() + 8 * rows * cols
+
+    def run(mask):
+        call("sp_refine_support", ptr(avg_t), rows, cols, ptr(k) if mask is None else None,
+             k.data_ptr() + 8 * (rows if rows != cols else 0) if mask is None else None, ptr(mask),
+             float(local_threshold), float(global_threshold), 1 if kill_weakest else 0, ptr(work),
+             nbytes.value, ptr(out), refined_ptr, stream_ptr())
+
+    run(None)  # the blur, under way while the host makes the mask
+    run(torch.from_numpy(np.ascontiguousarray(masking.inside(support)).view(np.uint8)).to(dev))
+    host = out.cpu().numpy()
+    blurred = host[:8 * rows * cols].view(np.float64).reshape(rows, cols)
+    refined = host[8 * rows * cols:].view(np.float32).reshape(rows, cols)
+    return refined.astype(support.dtype if support.dtype.kind == "f" else np.int64, copy=False), blurred
 
 
 # the module function under a second name, for methods whose keyword

@@ -212,7 +212,9 @@ int sp_shrinkwrap(const void* avg_dev, int rows, int cols, const double* kr_dev,
 /* The same with the parts found on the device: mask_dev (bytes, rows*cols, non-zero
  * inside the support) is split into its connected parts (8 neighbours, periodic; a
  * pixel with no neighbour in the mask is an empty part).  work_dev: scratch of
- * sp_refine_workspace_size bytes, 8-byte aligned. */
+ * sp_refine_workspace_size bytes, 8-byte aligned.  Without mask_dev only the blur is
+ * made; without kr_dev and kc_dev blurred_dev is taken as it is, so that the blur can
+ * run while a caller prepares the mask. */
 int sp_refine_workspace_size(int rows, int cols, size_t* bytes);
 int sp_refine_support(const void* avg_dev, int rows, int cols, const double* kr_dev,
                       const double* kc_dev, const unsigned char* mask_dev, double local_t,
