@@ -88,11 +88,11 @@ __global__ void __launch_bounds__(kThreads) fft_cols_kernel(const float2* in,
 // then a column of its own, loaded, transformed and added up in registers with
 // no barrier wider than the line.  128 frames of 180^2 at N = 512: 40 us of rows
 // (store-bound: 94 MB in 64-byte pieces), 71 us of columns (instruction issue)
-// and 12 us to add the partial sums up, against 435 us for embedding, two
+// and 6 us to add the partial sums up, against 435 us for embedding, two
 // passes over the planes and an accumulation; columns interleaved in a CTA,
-// with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 66 us, from
-// 128 us.  Radix 32 (two stages at 512) made the columns 65 us but changed the
-// transforms' rounding.
+// with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 53 us (rows
+// 14, columns 32, sums 5), from 128 us.  Radix 32 (two stages at 512) made the
+// columns 65 us but changed the transforms' rounding.
 // ---------------------------------------------------------------------------
 struct EmbedArgs {
   const float2* src;
@@ -240,6 +240,17 @@ struct EmbedRowsOp {
 __host__ __device__ constexpr int embed_group_cols(int N) {
   return lines_per_item_t(N, embed_e(N), kEmbedThreads);
 }
+// An Op's goal values of a group's columns are staged row by row (read straight
+// by the columns' threads, every value is a sector of its own: 39 us for 37
+// frames at 512, 32 staged; kept in shared memory instead of each thread's
+// registers 35).  Pitch: the 32 / L rows of a warp's store on different banks.
+__host__ __device__ constexpr int embed_goal_pitch(int N) {
+  return N + (embed_group_cols(N) < 32 ? 32 / embed_group_cols(N) : 1);
+}
+template <int N, class Op>
+constexpr int embed_goal_floats() {
+  return Op::kGoal ? embed_group_cols(N) * embed_goal_pitch(N) : 0;
+}
 template <int N, class Op>
 __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_kernel(EmbedArgs a, Op op,
                                                                                   int run) {
@@ -264,10 +275,18 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
     float2* p = a.dst + (size_t)f0 * N * N + (size_t)col * N + t;
     typename Op::Acc acc[E];
     typename Op::Pixel px[E];
+    float* goal = reinterpret_cast<float*>(tw + tw_stage_total(N, E));
+    constexpr int GP = embed_goal_pitch(N);
+    if constexpr (Op::kGoal) {
+      __syncthreads();  // the previous group's values are read
+      for (int k = threadIdx.x; k < N * L; k += kEmbedThreads)
+        goal[k % L * GP + k / L] = op.goal[(size_t)(k / L) * N + g * L + k % L];
+      __syncthreads();
+    }
 #pragma unroll
     for (int i = 0; i < E; ++i) {
       acc[i] = typename Op::Acc{};
-      px[i] = op.pixel((size_t)(t + i * T) * N + col);
+      if constexpr (Op::kGoal) px[i] = op.pixel(goal[(active ? lc : 0) * GP + t + i * T]);
     }
     for (int f = 0; f < nf; ++f) {
       const float2* q = p + (size_t)f * N * N;
@@ -321,7 +340,7 @@ struct PhasorSum {
   using Acc = float2;
   __device__ static float2 store(float2 x) { return x; }
   __device__ static void plus(float2& a, float2 b) { a.x += b.x, a.y += b.y; }
-  __device__ Pixel pixel(size_t) const { return {}; }
+  static constexpr bool kGoal = false;
   __device__ __forceinline__ static bool plain(float p2) { return p2 > 1e-30f && p2 < 1e30f; }
   // adds the summand unless its magnitude needs add_odd; whether it did
   __device__ __forceinline__ bool add(float2& acc, float2 v, Pixel) const {
@@ -356,10 +375,8 @@ struct RftfSum {
   using Acc = float;
   __device__ static float2 store(float x) { return make_float2(x, 0.f); }
   __device__ static void plus(float& a, float b) { a += b; }
-  __device__ Pixel pixel(size_t k) const {
-    const float g = goal[k];
-    return {g, 1.f / (g * g)};
-  }
+  static constexpr bool kGoal = true;
+  __device__ static Pixel pixel(float g) { return {g, 1.f / (g * g)}; }
   __device__ __forceinline__ bool add(float& acc, float2 v, Pixel p) const {
     const float p2 = v.x * v.x + v.y * v.y;
     const float d1 = p.g - (p2 > 0.f && p2 < 3e38f ? p2 * rsqrtf(p2) : p2);
@@ -378,7 +395,8 @@ template <int N, class Op>
 cudaError_t embed_sum_t(const EmbedArgs& a, const Op& op, int* run, int* group_cols, int n_sms,
                         cudaStream_t st) {
   constexpr int E = embed_e(N), LC = embed_group_cols(N);
-  const int sc = (LC * padk(N, pad_shift(E)) + tw_stage_total(N, E)) * (int)sizeof(float2);
+  const int sc = (LC * padk(N, pad_shift(E)) + tw_stage_total(N, E)) * (int)sizeof(float2) +
+                 embed_goal_floats<N, Op>() * (int)sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(embed_cols_sum_kernel<N, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, sc);
   if (e != cudaSuccess) return e;
   const int64_t total = (int64_t)(N / LC) * a.n, slots = (int64_t)embed_ctas(N) * n_sms;
