@@ -87,10 +87,11 @@ __global__ void __launch_bounds__(kThreads) fft_cols_kernel(const float2* in,
 // so that a column is contiguous; in the column kernel every line of a CTA is
 // then a column of its own, loaded, transformed and added up in registers with
 // no barrier wider than the line.  128 frames of 180^2 at N = 512: 40 us of rows
-// (store-bound: 94 MB in 64-byte pieces), 71 us of columns (instruction issue)
-// and 6 us to add the partial sums up, against 435 us for embedding, two
-// passes over the planes and an accumulation; columns interleaved in a CTA,
-// with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 53 us (rows
+// (shared-memory wavefronts, 78% of their rate: two exchanges, the twiddles and
+// the strips' transposition; with its stores in contiguous pieces 37), 71 us of
+// columns (instruction issue) and 6 us to add the partial sums up, against 435
+// us for embedding, two passes over the planes and an accumulation; columns
+// interleaved in a CTA, with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 53 us (rows
 // 14, columns 32, sums 5), from 128 us.  Radix 32 (two stages at 512) made the
 // columns 65 us but changed the transforms' rounding.
 // ---------------------------------------------------------------------------
