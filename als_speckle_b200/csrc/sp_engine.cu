@@ -416,16 +416,26 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
 // 460 / 402; 16 x 512^2 + 4 x 1024^2 136 / 118; 16 x 256^2 + 8 x 512^2 + 3 x 1024^2 +
 // 2048^2 245 / 201 alone, 219 / 176 with calls on three streams (the 256^2
 // trials in a line of their own: 187 and 210).  Everything in one line is slower
-// where sizes leave SMs idle (512^2 + 1024^2: 29 / 34).  The joins are made even
-// after a failed launch, so a capture never ends with unjoined work.
+// where sizes leave SMs idle (512^2 + 1024^2: 29 / 34).  Beyond kLineRounds
+// rounds in all, what the overlap saves at the ends of passes is small, and sizes
+// that run side by side use memory and issue slots more evenly, so each gets a
+// line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds 1775 / 1779,
+// 182 rounds (70 x 1024^2 + 35 x 2048^2) 3428 / 3483, 214 rounds 3840 / 3911.
+// The joins are made even after a failed launch, so a capture never ends with
+// unjoined work.
+constexpr double kLineRounds = 90;
 static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, const Item* items,
                         const int2* jobs, const float2* tw, ForkPool* P, cudaStream_t st) {
   if (P == nullptr || segs.size() == 1)
     return launch_line(segs, slots, items, jobs, tw, false, st);
-  double work = 0;
-  for (const Segment& sg : segs) work += sg.work;
+  double work = 0, rounds = 0;
+  for (const Segment& sg : segs) {
+    work += sg.work;
+    rounds += sg.rounds;
+  }
+  const bool apart = rounds > kLineRounds;
   auto shared = [&](const Segment& sg) {
-    return sg.rounds > 1.0 || (sg.rounds > 0.75 && sg.work < 0.2 * work);
+    return !apart && (sg.rounds > 1.0 || (sg.rounds > 0.75 && sg.work < 0.2 * work));
   };
   std::vector<std::vector<Segment>> lines(1);  // [0] on `st`
   for (const Segment& sg : segs)
@@ -446,9 +456,9 @@ static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, con
       break;
     }
     forked = i + 1;
-    if (rc == SP_OK) rc = launch_line(lines[i + 1], slots, items, jobs, tw, true, P->streams[i]);
+    if (rc == SP_OK) rc = launch_line(lines[i + 1], slots, items, jobs, tw, !apart, P->streams[i]);
   }
-  if (rc == SP_OK) rc = launch_line(lines[0], slots, items, jobs, tw, n_aux > 0, st);
+  if (rc == SP_OK) rc = launch_line(lines[0], slots, items, jobs, tw, n_aux > 0 && !apart, st);
   for (int i = 0; i < forked; ++i) {
     const cudaError_t e1 = cudaEventRecord(P->events[1 + i], P->streams[i]);
     const cudaError_t e2 = cudaStreamWaitEvent(st, P->events[1 + i], 0);

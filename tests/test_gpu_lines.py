@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
     ((512, 10, 5, "hio"), (1024, 3, 7, "raar")),
     ((256, 40, 4, "dm"), (512, 9, 6, "hio"), (1024, 2, 3, "dm"), (2048, 1, 5, "er")),
     ((128, 2, 9, "hio"), (512, 1, 4, "raar"), (2048, 1, 3, "hio")),
-    ((256, 38, 6, "er"), (512, 9, 4, "ipsf"), (1024, 2, 5, "hio"))])
+    ((256, 38, 6, "er"), (512, 9, 4, "ipsf"), (1024, 2, 5, "hio")),
+    # so many rounds that every size gets a line of its own
+    ((256, 20, 4, "dm"), (1024, 40, 2, "hio"), (2048, 18, 3, "raar"))])
 def test_mixed_lines_match_alone(mix):
     import torch
     from als_speckle_b200.engine import Engine, TrialSpec
