@@ -24,7 +24,12 @@ struct PassArgs {
 // starts at once, on the SMs that the previous kernel's last round leaves idle,
 // and waits after its first item.  Either way it lets the next kernel in only
 // after its wait, so when a kernel starts everything before its predecessor is
-// complete.  With `late`, each CTA lets it in only when it begins its last item:
+// complete: the planes that an early first item reads are in L2.  What the wait
+// would add is that this SM sees them so: the column pass's 8-byte copies go
+// through L1, which may still hold the lines that an earlier tick's pass read
+// there.  So an early start makes a device-scope fence first, which drops them;
+// nothing that runs beside the kernel writes these planes, so what is read from
+// then on is what L2 holds.  With `late`, each CTA lets it in only when it begins its last item:
 // CTAs let in earlier hold SMs that a concurrent line of launches could use (20 x
 // 512^2 beside 12 x 256^2: 86 against 91 us per iteration; alone, earlier is better,
 // 4 x 2048^2 266 against 268).
@@ -33,7 +38,10 @@ struct PassArgs {
 // 2%).
 template <bool LINE>
 __device__ __forceinline__ void chain_start(const PassArgs& a) {
-  if (LINE && a.overlap) return;
+  if (LINE && a.overlap) {
+    __threadfence();
+    return;
+  }
   pdl_wait_prev();
   if (!(LINE && a.late)) pdl_allow_next();
 }

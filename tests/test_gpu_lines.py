@@ -67,3 +67,44 @@ def test_mixed_lines_match_alone(mix):
     for a, b in zip(*batches):
         np.testing.assert_array_equal(a, b)
     eng.close()
+
+
+@pytest.mark.parametrize("mix", [
+    # several rounds of the SMs each, so that a size's pass starts early, on SMs
+    # that read its planes a tick ago: 8-byte copies through L1 at every size but 512
+    ((256, 40, 30, "hio"), (1024, 4, 30, "raar")),
+    ((1024, 3, 24, "hio"), (2048, 1, 24, "hio")),
+    ((256, 24, 24, "dm"), (512, 12, 24, "hio"), (1024, 3, 24, "er"))])
+def test_early_passes_read_what_the_last_tick_wrote(mix):
+    """Every trial of a long mixed batch, bit for bit, against its size alone
+    (one size in a call never starts early)."""
+    import torch
+    from als_speckle_b200.engine import Engine, TrialSpec
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    specs = []
+    for N, count, its, alg in mix:
+        S = torch.zeros((N, N), device="cuda")
+        S[N // 8:N // 2, N // 4:N // 2 + 3] = 1
+        M = 30 * torch.rand((N, N), generator=g, device="cuda")
+        for _ in range(count):
+            specs.append(dict(modulus=M, support=S, iterations=its, order=((alg, its),), beta=0.9,
+                              random_phase=True, seed=6, trial=len(specs)))
+
+    def solve(eng, sel):
+        sp = [TrialSpec(psi=torch.zeros(tuple(s["modulus"].shape), dtype=torch.complex64, device="cuda"), **s)
+              for s in sel]
+        for _ in range(2):
+            eng.solve(sp)
+        torch.cuda.synchronize()
+        return [s.psi for s in sp]
+
+    eng = Engine(use_graph=False)
+    mixed = solve(eng, specs)
+    alone, k = [], 0
+    for _, count, _, _ in mix:
+        alone += solve(eng, specs[k:k + count])
+        k += count
+    for k, (a, b) in enumerate(zip(mixed, alone)):
+        assert torch.equal(torch.view_as_real(a), torch.view_as_real(b)), k
+    eng.close()
