@@ -278,11 +278,17 @@ __global__ void __launch_bounds__(kRegThreads, 4) reg_upsample_cols_kernel(
 template <int MQ>
 static cudaError_t reg_upsample(const RegArgs& a, int N, unsigned long long* best_up, cudaStream_t st) {
   constexpr int rows = reg_tile_rows(MQ);
-  const int smem = (int)(sizeof(float4) * rows * kRegK + sizeof(float2) * 2 * (size_t)kRegK * a.M);
+  const auto bytes = [](int M) {
+    return (int)(sizeof(float4) * rows * kRegK + sizeof(float2) * 2 * (size_t)kRegK * M);
+  };
+  // (the limit is the process's: that of the instantiation's largest M, whatever
+  // this call's is, so that threads with other sizes do not lower it between this
+  // and the launch)
+  const int smem = bytes(a.M), most = bytes(32 * MQ);
   cudaError_t e = cudaFuncSetAttribute(reg_upsample_rows_kernel<MQ>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(reg_upsample_cols_kernel<MQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  e = cudaFuncSetAttribute(reg_upsample_cols_kernel<MQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e != cudaSuccess) return e;
   reg_upsample_rows_kernel<MQ><<<dim3((N + rows - 1) / rows, a.n), kRegThreads, smem, st>>>(
       a.F, a.Rf, a.W, a.best, a.X, N, a.M);

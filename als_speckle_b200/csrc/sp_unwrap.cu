@@ -330,11 +330,14 @@ extern "C" int sp_unwrap(const float* in_dev, int N, int r_in, int r_out, double
     spline_cols_kernel<<<nb, tb, 0, st>>>(in_dev, work_dev, N);
   SP_CUDA_TRY(cudaGetLastError());
   if (seg) {
-    const size_t row_bytes = (size_t)(N + N / kSeg + 1) * 2 * sizeof(double);
+    const auto bytes = [](int n) { return (size_t)(n + n / kSeg + 1) * 2 * sizeof(double); };
+    const size_t row_bytes = bytes(N);
     const int warps = row_bytes * 4 <= 64 * 1024 ? 4 : 1;  // rows per CTA
+    // (the limit is the process's: the largest call's, whatever this one needs, so
+    // that threads with other sizes do not lower it before this launch)
     SP_CUDA_TRY(cudaFuncSetAttribute(spline_rows_seg_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(row_bytes * warps)));
+                                     (int)bytes(kSegRowMax)));
     spline_rows_seg_kernel<<<(N + warps - 1) / warps, 32 * warps, row_bytes * warps, st>>>(work_dev, N);
   } else {
     spline_rows_kernel<<<nb, tb, 0, st>>>(work_dev, N);
