@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
     typename Op::Pixel px[E];
     float* goal = reinterpret_cast<float*>(tw + tw_stage_total(N, E));
     constexpr int GP = embed_goal_pitch(N);
+    bool odd_px = false;  // a pixel whose summands need add_odd
     if constexpr (Op::kGoal) {
       __syncthreads();  // the previous group's values are read
       for (int k = threadIdx.x; k < N * L; k += kEmbedThreads)
@@ -288,6 +289,7 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
     for (int i = 0; i < E; ++i) {
       acc[i] = typename Op::Acc{};
       if constexpr (Op::kGoal) px[i] = op.pixel(goal[(active ? lc : 0) * GP + t + i * T]);
+      odd_px |= Op::odd(px[i]);
     }
     for (int f = 0; f < nf; ++f) {
       const float2* q = p + (size_t)f * N * N;
@@ -297,8 +299,13 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
         v[i] = (active && t + i * T < a.rows) ? __ldcg(q + i * T) : make_float2(0.f, 0.f);
       fft_line<N, E, -1>(v, lay, sync, active, t, tw);
       bool odd = false;
+      if (odd_px) {
 #pragma unroll
-      for (int i = 0; i < E; ++i) odd |= !op.add(acc[i], v[i], px[i]);
+        for (int i = 0; i < E; ++i) Op::add_odd(acc[i], v[i], px[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < E; ++i) odd |= !op.add(acc[i], v[i], px[i]);
+      }
       if (odd) {
 #pragma unroll 1
         for (int i = 0; i < E; ++i) {
@@ -309,12 +316,13 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
 #pragma unroll
           for (int k = 1; k < E; ++k)
             if (k == i) x = v[k], y = px[k];
-          op.add_odd(z, x, y);
+          Op::add_odd(z, x, y);
 #pragma unroll
           for (int k = 0; k < E; ++k)
             if (k == i) Op::plus(acc[k], z);
         }
       }
+      if constexpr (T > 32) __syncwarp();  // the next line barrier takes whole warps
     }
     if (active) {
 #pragma unroll
@@ -342,6 +350,7 @@ struct PhasorSum {
   __device__ static float2 store(float2 x) { return x; }
   __device__ static void plus(float2& a, float2 b) { a.x += b.x, a.y += b.y; }
   static constexpr bool kGoal = false;
+  __device__ __forceinline__ static bool odd(Pixel) { return false; }
   __device__ __forceinline__ static bool plain(float p2) { return p2 > 1e-30f && p2 < 1e30f; }
   // adds the summand unless its magnitude needs add_odd; whether it did
   __device__ __forceinline__ bool add(float2& acc, float2 v, Pixel) const {
@@ -353,7 +362,7 @@ struct PhasorSum {
     acc.y = ok ? fmaf(v.y, r, acc.y) : acc.y;
     return ok;
   }
-  __device__ void add_odd(float2& acc, float2 v, Pixel) const {
+  __device__ static void add_odd(float2& acc, float2 v, Pixel) {
     if (plain(v.x * v.x + v.y * v.y)) return;
     const float h = hypotf(v.x, v.y);
     if (h > 0.f) {
@@ -364,10 +373,11 @@ struct PhasorSum {
 };
 
 // 1/sqrt(1 + (g - |F|)^2 / g^2) summed (phasing_rftf_accumulate.cl), g the goal
-// modulus.  1/sqrt(x) by the reciprocal square root and one Newton step;
-// nothing needs a slow form (at g = 0 the quotient is infinite, or NaN for
-// F = 0 too, as in the division; a square past the range leaves |F| infinite
-// and the summand 0, as a square root would).
+// modulus.  1/sqrt(x) by the reciprocal square root and one Newton step.  At g = 0
+// the quotient is infinite, or NaN for F = 0 too, as in the division; a square past
+// the range leaves |F| infinite and the summand 0, as a square root would.  From
+// g = 9.2e18 on 1/g^2 is below the normal range (and flushed): a thread with such a
+// pixel (`odd`) takes the quotient itself.
 struct RftfSum {
   const float* goal;
   struct Pixel {
@@ -378,16 +388,23 @@ struct RftfSum {
   __device__ static void plus(float& a, float b) { a += b; }
   static constexpr bool kGoal = true;
   __device__ static Pixel pixel(float g) { return {g, 1.f / (g * g)}; }
-  __device__ __forceinline__ bool add(float& acc, float2 v, Pixel p) const {
+  __device__ __forceinline__ static bool odd(Pixel p) { return p.inv == 0.f; }
+  __device__ __forceinline__ static float misfit(float2 v, Pixel p) {
     const float p2 = v.x * v.x + v.y * v.y;
-    const float d1 = p.g - (p2 > 0.f && p2 < 3e38f ? p2 * rsqrtf(p2) : p2);
+    return p.g - (p2 > 0.f && p2 < 3e38f ? p2 * rsqrtf(p2) : p2);
+  }
+  __device__ __forceinline__ bool add(float& acc, float2 v, Pixel p) const {
+    const float d1 = misfit(v, p);
     const float x = 1.f + (d1 * d1) * p.inv;
     float r = rsqrtf(x);
     if (x < 1e30f) r = r * fmaf(-0.5f * x * r, r, 1.5f);
     acc += r;
     return true;
   }
-  __device__ void add_odd(float&, float2, Pixel) const {}
+  __device__ __forceinline__ static void add_odd(float& acc, float2 v, Pixel p) {
+    const float d1 = misfit(v, p);
+    acc += 1.f / sqrtf(1.f + (d1 * d1) / (p.g * p.g));
+  }
 };
 
 // Row and column kernels of embedded frames; *run and *group_cols say where

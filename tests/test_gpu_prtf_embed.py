@@ -73,3 +73,23 @@ def test_rftf_of_extreme_magnitudes():
     got = gpu_rftf(None, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()).cpu().numpy()
     # frame 1: F = 0, summand 1/sqrt(2)
     assert np.allclose(got, 0.5 / np.sqrt(2.0), rtol=1e-6)
+
+
+@pytest.mark.parametrize("N", [32, 1024])
+@pytest.mark.parametrize("goal", [9e18, 9.3e18, 1e19, 1.8e19])
+def test_rftf_of_large_goals(goal, N):
+    """Goals whose square's reciprocal lies below the float range (from 9.2e18 on)
+    beside ordinary ones, F the same everywhere (a frame that is one point).  A
+    summand is a few roundings: 1e-6."""
+    import torch
+    from als_speckle_b200.phasing import gpu_rftf
+    x = np.zeros((3, 4, 4), np.complex64)
+    x[:, 0, 0] = [4e18, 1e18, 1.2e19]
+    g = np.full((N, N), goal, np.float32)
+    g[::3, ::2] = 3e18
+    g[5, 7] = 0
+    got = gpu_rftf(None, torch.from_numpy(x).cuda(), torch.from_numpy(g).cuda()).cpu().numpy()
+    with np.errstate(divide="ignore"):
+        want = np.mean([1 / np.sqrt(1 + (g.astype(np.float64) - f) ** 2 / g.astype(np.float64) ** 2)
+                        for f in np.abs(x[:, 0, 0]).astype(np.float64)], axis=0)
+    np.testing.assert_allclose(np.fft.ifftshift(got), want, rtol=1e-6, atol=1e-7)
