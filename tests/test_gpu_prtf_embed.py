@@ -93,3 +93,19 @@ def test_rftf_of_large_goals(goal, N):
         want = np.mean([1 / np.sqrt(1 + (g.astype(np.float64) - f) ** 2 / g.astype(np.float64) ** 2)
                         for f in np.abs(x[:, 0, 0]).astype(np.float64)], axis=0)
     np.testing.assert_allclose(np.fft.ifftshift(got), want, rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("N,frames", [(32, 600), (64, 900), (256, 300)])
+def test_mean_of_many_frames(N, frames):
+    """Frames that are one point, whose transforms are the same everywhere: the
+    RFTF's summand is 1/sqrt(2), the PRTF's phasor a quarter turn's.  A summand is
+    good to 1.5 units of its last place and the means of equal ones, added up in
+    FP64 but for runs of a few, to little more: 4e-7 relative."""
+    import torch
+    from als_speckle_b200.phasing import gpu_rftf, prtf
+    x = torch.zeros((frames, 3, 2), dtype=torch.complex64, device="cuda")
+    x[:, 0, 0] = 1.2 + 1.6j
+    g = torch.ones((N, N), device="cuda")
+    got = gpu_rftf(None, x, g).cpu().numpy()
+    np.testing.assert_allclose(got, np.full((N, N), 1 / np.sqrt(2.0)), rtol=4e-7)
+    np.testing.assert_allclose(prtf(x, N=N).cpu().numpy(), np.ones((N, N)), rtol=4e-7)
