@@ -102,13 +102,13 @@ struct EmbedArgs {
   const float2* tw;
 };
 
-constexpr int kEmbedThreads = 128;  // CTAs of the column kernel
+// threads of the column kernel's CTAs: a line of 16 values a thread
+__host__ __device__ constexpr int embed_threads(int N) { return N >= 4096 ? 256 : 128; }
 // values per thread: those of sp_fft2, so that the transforms are its bit for
-// bit (where F is nearly 0 its phasor amplifies any change of rounding), but
-// for columns of 4096 points, which would need 256 threads
-__host__ __device__ constexpr int embed_e(int N) { return N >= 4096 ? 32 : (N < 16 ? N : 16); }
+// bit (where F is nearly 0 its phasor amplifies any change of rounding)
+__host__ __device__ constexpr int embed_e(int N) { return N < 16 ? N : 16; }
 // resident CTAs per SM it is compiled for
-__host__ __device__ constexpr int embed_ctas(int N) { return embed_e(N) > 16 ? 3 : 5; }
+__host__ __device__ constexpr int embed_ctas(int N) { return embed_threads(N) > 128 ? 2 : 5; }
 
 // ---------------------------------------------------------------------------
 // Lines of planes transformed one by one: a CTA takes L lines of one plane, T
@@ -239,7 +239,7 @@ struct EmbedRowsOp {
 // sums of group g lie in planes f with f = 0 or (g n + f) % run = 0 (see
 // for_each_sum).  `Op` maps (F, pixel) to the summand.
 __host__ __device__ constexpr int embed_group_cols(int N) {
-  return lines_per_item_t(N, embed_e(N), kEmbedThreads);
+  return lines_per_item_t(N, embed_e(N), embed_threads(N));
 }
 // An Op's goal values of a group's columns are staged row by row (read straight
 // by the columns' threads, every value is a sector of its own: 39 us for 37
@@ -253,7 +253,7 @@ constexpr int embed_goal_floats() {
   return Op::kGoal ? embed_group_cols(N) * embed_goal_pitch(N) : 0;
 }
 template <int N, class Op>
-__global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_kernel(EmbedArgs a, Op op,
+__global__ void __launch_bounds__(embed_threads(N), embed_ctas(N)) embed_cols_sum_kernel(EmbedArgs a, Op op,
                                                                                   int run) {
   constexpr int E = embed_e(N), T = N / E, L = embed_group_cols(N);
   constexpr int SH = pad_shift(E);
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kEmbedThreads, embed_ctas(N)) embed_cols_sum_k
     bool odd_px = false;  // a pixel whose summands need add_odd
     if constexpr (Op::kGoal) {
       __syncthreads();  // the previous group's values are read
-      for (int k = threadIdx.x; k < N * L; k += kEmbedThreads)
+      for (int k = threadIdx.x; k < N * L; k += embed_threads(N))
         goal[k % L * GP + k / L] = op.goal[(size_t)(k / L) * N + g * L + k % L];
       __syncthreads();
     }
@@ -422,7 +422,7 @@ cudaError_t embed_sum_t(const EmbedArgs& a, const Op& op, int* run, int* group_c
   *group_cols = LC;
   e = launch_lines<N, -1>(EmbedRowsOp{a.src, a.dst, a.n, a.rows, a.cols}, a.tw, n_sms, st);
   if (e != cudaSuccess) return e;
-  embed_cols_sum_kernel<N, Op><<<(int)((total + *run - 1) / *run), kEmbedThreads, sc, st>>>(a, op, *run);
+  embed_cols_sum_kernel<N, Op><<<(int)((total + *run - 1) / *run), embed_threads(N), sc, st>>>(a, op, *run);
   return cudaGetLastError();
 }
 

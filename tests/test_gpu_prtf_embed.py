@@ -109,3 +109,23 @@ def test_mean_of_many_frames(N, frames):
     got = gpu_rftf(None, x, g).cpu().numpy()
     np.testing.assert_allclose(got, np.full((N, N), 1 / np.sqrt(2.0)), rtol=4e-7)
     np.testing.assert_allclose(prtf(x, N=N).cpu().numpy(), np.ones((N, N)), rtol=4e-7)
+
+
+@pytest.mark.parametrize("N,rows,cols", [(8, 5, 8), (64, 40, 33), (512, 180, 181), (2048, 300, 77), (4096, 300, 321)])
+def test_phasors_of_the_standalone_transform(N, rows, cols):
+    """One frame's phasors are those of sp_fft2's transform of the embedded frame,
+    to the phasor's own few roundings (3e-7): the transforms are the same bits, where
+    another order of operations would show wherever F is small."""
+    import torch
+    from als_speckle_b200._lib import call, ptr, stream_ptr
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    x = torch.view_as_complex(torch.randn((rows, cols, 2), generator=g, device="cuda"))
+    F = torch.zeros((N, N), dtype=torch.complex64, device="cuda")
+    F[:rows, :cols] = x
+    call("sp_fft2", ptr(F), ptr(F), N, 1, 0, stream_ptr())
+    got = torch.zeros((N, N), dtype=torch.complex64, device="cuda")
+    work = torch.empty((1, N, N), dtype=torch.complex64, device="cuda")
+    call("sp_prtf_phasors", ptr(x), 1, rows, cols, N, ptr(work), ptr(got), stream_ptr())
+    F = F.to(torch.complex128)
+    assert (got.to(torch.complex128) - F / F.abs()).abs().max().item() < 3e-7
