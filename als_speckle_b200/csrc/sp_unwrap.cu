@@ -74,76 +74,122 @@ __device__ void bspline3_line(const T* in, double* out, int n, long stride) {
 }
 
 // Lines of kSegMin and more are prefiltered in segments of kSeg values, one
-// thread each: the recursions forget their past by |z| = 0.268 a step, so a
-// thread that starts kWarm = 32 steps before its segment (after it, for the
-// anti-causal one) from zero is off by |z|^32 = 5e-19 of the line's scale,
-// below FP64's rounding, and the exact boundary sums need 64 terms only.  One
-// thread per line (kept for short and very long lines) is a chain of 4 n
+// thread each.  The recursions are linear, so a segment runs from zero first,
+// and what comes in from before it (after it, for the anti-causal one) is the
+// sum of the other segments' ends, each times z^kSeg per segment between:
+// kFar = 12 of them, beyond which z^(kSeg kFar) = 1e-110 of a value is below
+// any sample's last place (float32 spans 4e-84), however far apart the map's
+// values lie.  A warm-up of 32 steps in place of the carries dropped 5e-19 of
+// the line's largest value, which showed next to a value 1e15 times the others.
+// One thread per line (kept for short and very long lines) is a chain of 4 n
 // dependent FP64 steps on n threads: at 512 lines of 512 it took 238 us for
-// the columns and 247 us for the rows; the segments take 8 and 7 us.
-constexpr int kSeg = 16, kWarm = 32, kSegMin = 128;
-constexpr int kSegRowMax = 8192;  // longest row staged in shared memory
+// the columns and 247 us for the rows; the segments take 6 and 7 us (as the warm-ups did, 7 and 6; 5% more from 4096 on).
+constexpr int kSeg = 16, kFar = 12, kSegMin = 128;
+constexpr int kSegMax = 8192;  // longest row staged in shared memory
 
-// the causal recursion's first value of a line of n >= kSegMin samples,
-// p[0] = 6 sum_k z^k x[k] (the mirrored terms carry z^(n-1) < 1e-70)
+constexpr double zpow(int n) { return n == 0 ? 1.0 : kZ3 * zpow(n - 1); }
+constexpr double kZSeg = zpow(kSeg);
+
+// sum_{k = 1}^{kFar} z^(kSeg (k-1)) at(k), as far as there are `n` of them
 template <class F>
-__device__ __forceinline__ double bspline3_first(F&& x) {
+__device__ __forceinline__ double far_sum(int n, F&& at) {
   double s = 0.0;
-#pragma unroll 16
-  for (int k = 63; k >= 0; --k) s = x(k) + kZ3 * s;
-  return kGain3 * s;
+  for (int k = n < kFar ? n : kFar; k >= 1; --k) s = at(k) + kZSeg * s;
+  return s;
 }
 
-// Columns, thread (column j, segment): p in registers over the segment and
-// the warm-up of the way back; the map is only read and c only written, so
-// segments are independent.
-__global__ void __launch_bounds__(128) spline_cols_seg_kernel(const float* __restrict__ in,
-                                                              double* __restrict__ c, int N) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s0 = blockIdx.y * kSeg;
-  if (j >= N) return;
-  const float* x = in + j;
+// What a line's length fixes: z^(n-1) and z^(length of the last segment).  The
+// causal recursion's first value is that of bspline3_line,
+//   6 sum_k z^k x[k] + z^(n-1) (p0[n-1] - 6 x[n-1]),
+// p0 the recursion from zero (its mirrored terms; 1 - z^(2n-2) is 1 here).
+struct SegLine {
+  double zn1, zlast;
+};
+
+// Columns: a CTA takes C neighbouring columns, thread (column, segment), the
+// segment's values in registers throughout.
+template <int C>
+__global__ void __launch_bounds__(512) spline_cols_seg_kernel(const float* __restrict__ in,
+                                                              double* __restrict__ c, int N,
+                                                              SegLine line) {
+  __shared__ double ends[512], heads[C * kFar];
+  const int S = blockDim.x / C, s = threadIdx.x / C, tx = threadIdx.x % C;
+  const int j = blockIdx.x * C + tx, col = j < N ? j : N - 1;
+  const int s0 = s * kSeg, n = N - s0 < kSeg ? N - s0 : kSeg;
+  const float* x = in + (size_t)s0 * N + col;
+  float v[kSeg];
+#pragma unroll
+  for (int i = 0; i < kSeg; ++i) v[i] = i < n ? x[(size_t)i * N] : 0.f;
+  double end = 0.0;
+#pragma unroll
+  for (int i = 0; i < kSeg; ++i)
+    if (i < n) end = kGain3 * (double)v[i] + kZ3 * end;
+  ends[s * C + tx] = end;
+  if (s < kFar) {
+    double head = 0.0;
+#pragma unroll
+    for (int i = kSeg - 1; i >= 0; --i) head = (double)v[i] + kZ3 * head;
+    heads[s * C + tx] = head;
+  }
+  __syncthreads();
   double prev = 0.0;
-  int k = s0 - kWarm;
-  if (k <= 0) {
-    prev = bspline3_first([&](int i) { return (double)x[(size_t)i * N]; });
-    k = 1;
+  if (s == 0) {
+    const double head = far_sum(S, [&](int k) { return heads[(k - 1) * C + tx]; });
+    const double tail = ends[(S - 1) * C + tx] +
+                        line.zlast * far_sum(S - 1, [&](int k) { return ends[(S - 1 - k) * C + tx]; });
+    prev = kGain3 * head + line.zn1 * (tail - kGain3 * (double)in[(size_t)(N - 1) * N + col]);
+    end = prev;
+#pragma unroll
+    for (int i = 1; i < kSeg; ++i) end = kGain3 * (double)v[i] + kZ3 * end;
+    ends[tx] = end;
   }
-#pragma unroll 16
-  for (; k < s0; ++k) prev = kGain3 * (double)x[(size_t)k * N] + kZ3 * prev;
+  __syncthreads();
+  if (s > 0) prev = far_sum(s, [&](int k) { return ends[(s - k) * C + tx]; });
   const double before = prev;  // p[s0 - 1]
-  double p[kSeg + kWarm];
+  double p[kSeg];
 #pragma unroll
-  for (int i = 0; i < kSeg + kWarm; ++i) {
-    const int q = s0 + i;
-    if (q > 0 && q < N) prev = kGain3 * (double)x[(size_t)q * N] + kZ3 * prev;
-    p[i] = prev;  // (q = 0: prev is p[0] already; past the end: p[N-1])
+  for (int i = 0; i < kSeg; ++i) {
+    if (s0 + i > 0 && i < n) prev = kGain3 * (double)v[i] + kZ3 * prev;
+    p[i] = prev;  // (s0 + i = 0: the first value itself)
   }
-  double next = 0.0;
+  // from the last segment's boundary value, or from `next` after the segment
+  auto back = [&](double next, auto&& put) {
 #pragma unroll
-  for (int i = kSeg + kWarm - 1; i >= 0; --i) {
-    const int q = s0 + i;
-    if (q < N - 1) {
-      next = kZ3 * (next - p[i]);
-    } else if (q == N - 1) {  // the anti-causal boundary value
-      next = (kZ3 / (kZ3 * kZ3 - 1.0)) * (p[i] + kZ3 * (i > 0 ? p[i - 1] : before));
+    for (int i = kSeg - 1; i >= 0; --i) {
+      if (s == S - 1 && i == n - 1)
+        next = (kZ3 / (kZ3 * kZ3 - 1.0)) * (p[i] + kZ3 * (i > 0 ? p[i > 0 ? i - 1 : 0] : before));
+      else if (i < n)
+        next = kZ3 * (next - p[i]);
+      put(i, next);
     }
-    if (i < kSeg && q < N) c[(size_t)q * N + j] = next;
-  }
+    return next;
+  };
+  __syncthreads();  // the causal ends are read
+  ends[s * C + tx] = back(0.0, [](int, double) {});
+  __syncthreads();
+  back(far_sum(S - 1 - s, [&](int k) { return ends[(s + k) * C + tx]; }), [&](int i, double next) {
+    if (i < n && j < N) c[(size_t)(s0 + i) * N + j] = next;
+  });
 }
 
-// Rows in place, one warp per row: the row and its causal values in shared
-// memory (one spare value per kSeg, so that lanes a segment apart fall on
-// different banks), segments dealt to the lanes.  A row with a value that is
-// not finite becomes NaN as a whole, as the unsegmented recursions make it
-// (unwrap_kernel does the same across rows).
-__device__ __forceinline__ int seg_pad(int k) { return k + k / kSeg; }
-__global__ void spline_rows_seg_kernel(double* __restrict__ c, int N) {
+// Rows in place, one warp per row: the row, its causal values and the segments'
+// ends in shared memory (one spare value per kSeg, so that lanes a segment
+// apart fall on different banks), segments dealt to the lanes.  A row with a
+// value that is not finite becomes NaN as a whole, as the unsegmented
+// recursions make it (unwrap_kernel does the same across rows).
+__host__ __device__ constexpr int seg_pad(int k) { return k + k / kSeg; }
+// doubles of shared memory for a row: inputs (then c), causal values, ends
+__host__ __device__ constexpr int seg_row_doubles(int n) {
+  return 2 * (seg_pad(n) + 1) + (n + kSeg - 1) / kSeg;
+}
+__global__ void spline_rows_seg_kernel(double* __restrict__ c, int N, SegLine line) {
   extern __shared__ double row_s[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int row = blockIdx.x * (blockDim.x >> 5) + w;
-  double* x = row_s + (size_t)w * (N + N / kSeg + 1) * 2;  // inputs, then c
-  double* p = x + (N + N / kSeg + 1);
+  double* x = row_s + (size_t)w * seg_row_doubles(N);
+  double* p = x + seg_pad(N) + 1;
+  double* ends = p + seg_pad(N) + 1;
+  const int S = (N + kSeg - 1) / kSeg;
   if (row >= N) return;
   double* g = c + (size_t)row * N;
   bool bad = false;
@@ -157,36 +203,67 @@ __global__ void spline_rows_seg_kernel(double* __restrict__ c, int N) {
     return;
   }
   __syncwarp();
-  const double first = bspline3_first([&](int i) { return x[seg_pad(i)]; });
-  for (int s0 = lane * kSeg; s0 < N; s0 += 32 * kSeg) {
-    double prev = 0.0;
-    int k = s0 - kWarm;
-    if (k <= 0) {
-      prev = first;
-      k = 1;
-    }
+  for (int s = lane; s < S; s += 32) {
+    const int s0 = s * kSeg, e = s0 + kSeg < N ? s0 + kSeg : N;
+    double end = 0.0;
 #pragma unroll 8
-    for (; k < s0; ++k) prev = kGain3 * x[seg_pad(k)] + kZ3 * prev;
-    const int e = s0 + kSeg < N ? s0 + kSeg : N;
-    if (s0 == 0) p[0] = first;
+    for (int k = s0; k < e; ++k) end = kGain3 * x[seg_pad(k)] + kZ3 * end;
+    ends[s] = end;
+  }
+  double first = 0.0;  // lane s: segment s's share of the head sum
+  if (lane < kFar && lane < S) {
+    const int s0 = lane * kSeg, e = s0 + kSeg < N ? s0 + kSeg : N;
 #pragma unroll 8
-    for (; k < e; ++k) {
+    for (int k = e - 1; k >= s0; --k) first = x[seg_pad(k)] + kZ3 * first;
+    for (int k = 0; k < lane; ++k) first *= kZSeg;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+  __syncwarp();
+  if (lane == 0) {
+    const double tail =
+        ends[S - 1] + line.zlast * far_sum(S - 1, [&](int k) { return ends[S - 1 - k]; });
+    first = kGain3 * first + line.zn1 * (tail - kGain3 * x[seg_pad(N - 1)]);
+    double end = first;
+#pragma unroll
+    for (int k = 1; k < kSeg; ++k) end = kGain3 * x[seg_pad(k)] + kZ3 * end;
+    ends[0] = end;
+  }
+  __syncwarp();
+  for (int s = lane; s < S; s += 32) {
+    const int s0 = s * kSeg, e = s0 + kSeg < N ? s0 + kSeg : N;
+    double prev = s ? far_sum(s, [&](int k) { return ends[s - k]; }) : first;
+    if (s == 0) p[0] = first;
+#pragma unroll 8
+    for (int k = s ? s0 : 1; k < e; ++k) {
       prev = kGain3 * x[seg_pad(k)] + kZ3 * prev;
       p[seg_pad(k)] = prev;
     }
   }
-  __syncwarp();
-  for (int s0 = lane * kSeg; s0 < N; s0 += 32 * kSeg) {
-    const int e = s0 + kSeg < N ? s0 + kSeg : N;
+  __syncwarp();  // the causal ends are read, the causal values complete
+  for (int s = lane; s < S; s += 32) {
+    const int s0 = s * kSeg, e = s0 + kSeg < N ? s0 + kSeg : N;
     double next = 0.0;
-    int k = e + kWarm - 1;
-    if (k >= N - 1) {
+    int k = e - 1;
+    if (s == S - 1) {
       next = (kZ3 / (kZ3 * kZ3 - 1.0)) * (p[seg_pad(N - 1)] + kZ3 * p[seg_pad(N - 2)]);
-      if (e == N) x[seg_pad(N - 1)] = next;
-      k = N - 2;
+      x[seg_pad(k--)] = next;
     }
 #pragma unroll 8
-    for (; k >= e; --k) next = kZ3 * (next - p[seg_pad(k)]);
+    for (; k >= s0; --k) next = kZ3 * (next - p[seg_pad(k)]);
+    ends[s] = next;
+  }
+  __syncwarp();
+  for (int s = lane; s < S; s += 32) {
+    const int s0 = s * kSeg;
+    int k = s0 + kSeg - 1;
+    double next;
+    if (s == S - 1) {
+      k = N - 2;
+      next = x[seg_pad(N - 1)];
+    } else {
+      next = far_sum(S - 1 - s, [&](int i) { return ends[s + i]; });
+    }
 #pragma unroll 8
     for (; k >= s0; --k) {
       next = kZ3 * (next - p[seg_pad(k)]);
@@ -323,22 +400,28 @@ extern "C" int sp_unwrap(const float* in_dev, int N, int r_in, int r_out, double
            cy, cx, N, N);
   cudaStream_t st = as_stream(stream);
   const int tb = 128, nb = (N + tb - 1) / tb;
-  const bool seg = N >= kSegMin && N <= kSegRowMax;
-  if (seg)
-    spline_cols_seg_kernel<<<dim3(nb, (N + kSeg - 1) / kSeg), tb, 0, st>>>(in_dev, work_dev, N);
-  else
+  const bool seg = N >= kSegMin && N <= kSegMax;
+  const int S = (N + kSeg - 1) / kSeg;
+  const SegLine line{pow(kZ3, N - 1), pow(kZ3, N - (S - 1) * kSeg)};
+  if (!seg)
     spline_cols_kernel<<<nb, tb, 0, st>>>(in_dev, work_dev, N);
+  else if (4 * S <= 512)
+    spline_cols_seg_kernel<4><<<(N + 3) / 4, 4 * S, 0, st>>>(in_dev, work_dev, N, line);
+  else if (2 * S <= 512)
+    spline_cols_seg_kernel<2><<<(N + 1) / 2, 2 * S, 0, st>>>(in_dev, work_dev, N, line);
+  else
+    spline_cols_seg_kernel<1><<<N, S, 0, st>>>(in_dev, work_dev, N, line);
   SP_CUDA_TRY(cudaGetLastError());
   if (seg) {
-    const auto bytes = [](int n) { return (size_t)(n + n / kSeg + 1) * 2 * sizeof(double); };
-    const size_t row_bytes = bytes(N);
+    const size_t row_bytes = seg_row_doubles(N) * sizeof(double);
     const int warps = row_bytes * 4 <= 64 * 1024 ? 4 : 1;  // rows per CTA
     // (the limit is the process's: the largest call's, whatever this one needs, so
     // that threads with other sizes do not lower it before this launch)
     SP_CUDA_TRY(cudaFuncSetAttribute(spline_rows_seg_kernel,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)bytes(kSegRowMax)));
-    spline_rows_seg_kernel<<<(N + warps - 1) / warps, 32 * warps, row_bytes * warps, st>>>(work_dev, N);
+                                     (int)(seg_row_doubles(kSegMax) * sizeof(double))));
+    spline_rows_seg_kernel<<<(N + warps - 1) / warps, 32 * warps, row_bytes * warps, st>>>(work_dev, N,
+                                                                                           line);
   } else {
     spline_rows_kernel<<<nb, tb, 0, st>>>(work_dev, N);
   }
