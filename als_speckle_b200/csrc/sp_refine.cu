@@ -28,7 +28,8 @@ __global__ void __launch_bounds__(256) blur_kernel(const void* __restrict__ in,
   __shared__ double a[kSpan][kTile + 1];
   __shared__ double kk[kTaps];
   const int lines = ROWS ? rows : cols, n = ROWS ? cols : rows;
-  const int l0 = blockIdx.y * kTile, p0 = blockIdx.x * kTile;
+  const int across = (n - 1) / kTile + 1;  // (one grid dimension: any shape fits it)
+  const int l0 = blockIdx.x / across * kTile, p0 = blockIdx.x % across * kTile;
   const int lane = threadIdx.x % 32, u = 4 * (threadIdx.x / 32);  // positions p0 + u .. u + 3
   double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
   for (int j0 = 0; j0 < n; j0 += kTaps) {
@@ -117,7 +118,8 @@ __device__ __forceinline__ void part_join(int* parent, int a, int b) {
 
 __global__ void __launch_bounds__(256) parts_init_kernel(const unsigned char* __restrict__ mask,
                                                          int* __restrict__ parent, int rows, int cols) {
-  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
+  const int across = (cols - 1) / 32 + 1;
+  const int c = blockIdx.x % across * 32 + threadIdx.x, r = blockIdx.x / across * 8 + threadIdx.y;
   const bool in = r < rows && c < cols;
   const bool m = in && mask[(size_t)r * cols + c];
   const unsigned run = __ballot_sync(0xffffffffu, m);
@@ -129,7 +131,8 @@ __global__ void __launch_bounds__(256) parts_init_kernel(const unsigned char* __
 
 __global__ void __launch_bounds__(256) parts_join_kernel(const unsigned char* __restrict__ mask,
                                                          int* parent, int rows, int cols) {
-  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
+  const int across = (cols - 1) / 32 + 1;
+  const int c = blockIdx.x % across * 32 + threadIdx.x, r = blockIdx.x / across * 8 + threadIdx.y;
   if (r >= rows || c >= cols) return;
   const int i = r * cols + c;
   if (!mask[i]) return;
@@ -159,7 +162,8 @@ __global__ void __launch_bounds__(256) parts_join_kernel(const unsigned char* __
 __global__ void __launch_bounds__(256) parts_label_kernel(const unsigned char* __restrict__ mask,
                                                           int* parent, int* __restrict__ labels, int rows,
                                                           int cols) {
-  const int c = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
+  const int across = (cols - 1) / 32 + 1;
+  const int c = blockIdx.x % across * 32 + threadIdx.x, r = blockIdx.x / across * 8 + threadIdx.y;
   if (r >= rows || c >= cols) return;
   const int i = r * cols + c;
   int l = 0;
@@ -314,9 +318,10 @@ int grid_of(int64_t n) {
 
 cudaError_t launch_blur(const void* avg, int rows, int cols, const double* kr, const double* kc,
                         double* tmp, double* blurred, cudaStream_t st) {
-  const int tr = (rows + kTile - 1) / kTile, tc = (cols + kTile - 1) / kTile;
-  blur_kernel<true><<<dim3(tc, tr), 256, 0, st>>>(avg, kc, tmp, rows, cols);
-  blur_kernel<false><<<dim3(tr, tc), 256, 0, st>>>(tmp, kr, blurred, rows, cols);
+  const int64_t tiles = (int64_t)((rows - 1) / kTile + 1) * ((cols - 1) / kTile + 1);
+  if (tiles > INT32_MAX) return cudaErrorInvalidValue;
+  blur_kernel<true><<<(unsigned)tiles, 256, 0, st>>>(avg, kc, tmp, rows, cols);
+  blur_kernel<false><<<(unsigned)tiles, 256, 0, st>>>(tmp, kr, blurred, rows, cols);
   return cudaGetLastError();
 }
 
@@ -393,7 +398,7 @@ int sp_refine_support(const void* avg, int rows, int cols, const double* kr, con
   int* weakest = labels + total;
   if (kr) SP_CUDA_TRY(launch_blur(avg, rows, cols, kr, kc, tmp, blurred, st));
   if (!mask) return SP_OK;
-  const dim3 grid((cols + 31) / 32, (rows + 7) / 8), block(32, 8);
+  const dim3 grid((unsigned)(((int64_t)(cols - 1) / 32 + 1) * ((rows - 1) / 8 + 1))), block(32, 8);
   parts_init_kernel<<<grid, block, 0, st>>>(mask, parent, rows, cols);
   parts_join_kernel<<<grid, block, 0, st>>>(mask, parent, rows, cols);
   parts_label_kernel<<<grid, block, 0, st>>>(mask, parent, labels, rows, cols);

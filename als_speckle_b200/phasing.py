@@ -633,6 +633,11 @@ def _gaussian_1d_kernel(n, sigma):
     return g / g.sum()
 
 
+# supports of so many pixels and more have their parts labelled on the host (the
+# device numbers pixels in 32 bits)
+_HOST_PARTS = 2 ** 31 - 1
+
+
 def refine_support(support, average_mag, blur=3, local_threshold=.2, global_threshold=0,
                    kill_weakest=False):
     """Shrinkwrap (``phasing.py:1747-1815``): blur |avg| with a circular
@@ -661,20 +666,29 @@ def refine_support(support, average_mag, blur=3, local_threshold=.2, global_thre
     if rows != cols:
         k = np.concatenate((k, _gaussian_1d_kernel(cols, blur)))
     k = torch.from_numpy(k).to(dev)
-    nbytes = C.c_size_t(0)
-    call("sp_refine_workspace_size", rows, cols, C.byref(nbytes))
-    work = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
+    kr, kc = ptr(k), k.data_ptr() + 8 * (rows if rows != cols else 0)
     out = torch.empty(12 * rows * cols, dtype=torch.uint8, device=dev)  # blurred, then refined
     refined_ptr = out.data_ptr() + 8 * rows * cols
+    limits = float(local_threshold), float(global_threshold), 1 if kill_weakest else 0
+    if rows * cols < _HOST_PARTS:
+        nbytes = C.c_size_t(0)
+        call("sp_refine_workspace_size", rows, cols, C.byref(nbytes))
+        work = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
 
-    def run(mask):
-        call("sp_refine_support", ptr(avg_t), rows, cols, ptr(k) if mask is None else None,
-             k.data_ptr() + 8 * (rows if rows != cols else 0) if mask is None else None, ptr(mask),
-             float(local_threshold), float(global_threshold), 1 if kill_weakest else 0, ptr(work),
-             nbytes.value, ptr(out), refined_ptr, stream_ptr())
+        def run(kernels, mask):
+            call("sp_refine_support", ptr(avg_t), rows, cols, *kernels, ptr(mask), *limits, ptr(work),
+                 nbytes.value, ptr(out), refined_ptr, stream_ptr())
 
-    run(None)  # the blur, under way while the host makes the mask
-    run(torch.from_numpy(np.ascontiguousarray(masking.inside(support)).view(np.uint8)).to(dev))
+        run((kr, kc), None)  # the blur, under way while the host makes the mask
+        run((None, None),
+            torch.from_numpy(np.ascontiguousarray(masking.inside(support)).view(np.uint8)).to(dev))
+    else:
+        labels, n = masking.label_parts(support)
+        lab = torch.from_numpy(labels.astype(np.int32)).to(dev)
+        work = torch.empty(rows * cols + n + 1, dtype=torch.float64, device=dev)
+        sums = torch.empty(n + 1, dtype=torch.float64, device=dev)
+        call("sp_shrinkwrap", ptr(avg_t), rows, cols, kr, kc, ptr(lab), n, *limits, ptr(work), ptr(out),
+             refined_ptr, ptr(sums), stream_ptr())
     host = out.cpu().numpy()
     blurred = host[:8 * rows * cols].view(np.float64).reshape(rows, cols)
     refined = host[8 * rows * cols:].view(np.float32).reshape(rows, cols)

@@ -78,3 +78,38 @@ def test_refine_support_parts(kind, R, C):
             p = b[lab == lab[r, c]].max() * 0.7 if lab[r, c] else np.inf
             assert min(abs(b[r, c] - p) / p, abs(b[r, c] - b.max() * 0.3) / b.max()) < 1e-6
         assert len(diff) <= 2
+
+
+@pytest.mark.parametrize("shape", [(530000, 2), (2, 530000)])  # more tiles than a grid has in y
+def test_refine_support_of_long_thin_maps(shape):
+    """A constant map stays constant under the blur, so every pixel of the support is
+    above its thresholds and the support comes back, hole and all."""
+    import torch
+    from als_speckle_b200.phasing import refine_support
+    sup = np.ones(shape, np.float32)
+    sup.ravel()[1000:2000] = 0
+    avg = torch.full(shape, 2j, dtype=torch.complex64, device="cuda")
+    got, blurred = refine_support(sup, avg, blur=1.0, local_threshold=0.5)
+    assert np.allclose(blurred, 2.0, rtol=1e-12)
+    np.testing.assert_array_equal(got, sup)
+
+
+@pytest.mark.parametrize("kind", ["empty", "full", "rows", "singles", "spiral", "sparse", "percolating"])
+@pytest.mark.parametrize("R,C", [(33, 2), (97, 130), (340, 341)])
+def test_parts_from_the_host_match(kind, R, C, monkeypatch):
+    """The route of supports too large for the device's 32-bit pixel numbers (parts
+    labelled by the caller, sp_shrinkwrap) on small ones: the same blur bit for bit,
+    the same support."""
+    import torch
+    from als_speckle_b200 import phasing
+    rng = np.random.default_rng(R + C)
+    sup = _mask(kind, R, C, rng).astype(np.float64)
+    avg = torch.from_numpy((rng.random((R, C)) * 1j).astype(np.complex64)).cuda()
+    for kill in (False, True):
+        args = dict(blur=0.8, local_threshold=0.7, global_threshold=0.3, kill_weakest=kill)
+        got, blurred = phasing.refine_support(sup, avg, **args)
+        with monkeypatch.context() as m:
+            m.setattr(phasing, "_HOST_PARTS", 1)
+            host, b = phasing.refine_support(sup, avg, **args)
+        np.testing.assert_array_equal(b, blurred)
+        np.testing.assert_array_equal(host, got)
