@@ -689,9 +689,9 @@ def refine_support(support, average_mag, blur=3, local_threshold=.2, global_thre
         sums = torch.empty(n + 1, dtype=torch.float64, device=dev)
         call("sp_shrinkwrap", ptr(avg_t), rows, cols, kr, kc, ptr(lab), n, *limits, ptr(work), ptr(out),
              refined_ptr, ptr(sums), stream_ptr())
-    host = out.cpu().numpy()
-    blurred = host[:8 * rows * cols].view(np.float64).reshape(rows, cols)
-    refined = host[8 * rows * cols:].view(np.float32).reshape(rows, cols)
+    # (two arrays, so that keeping the support does not keep the blurred map too)
+    blurred = out[:8 * rows * cols].cpu().numpy().view(np.float64).reshape(rows, cols)
+    refined = out[8 * rows * cols:].cpu().numpy().view(np.float32).reshape(rows, cols)
     return refined.astype(support.dtype if support.dtype.kind == "f" else np.int64, copy=False), blurred
 
 

@@ -113,3 +113,20 @@ def test_parts_from_the_host_match(kind, R, C, monkeypatch):
             host, b = phasing.refine_support(sup, avg, **args)
         np.testing.assert_array_equal(b, blurred)
         np.testing.assert_array_equal(host, got)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int64])
+def test_results_hold_no_more_than_themselves(dtype):
+    """The refined support and the blurred map do not share memory: a program that
+    keeps a support for every round keeps 4 bytes a pixel of it."""
+    import torch
+    from als_speckle_b200.phasing import refine_support
+    n = 64
+    got = refine_support(np.ones((n, n), dtype), torch.ones((n, n), dtype=torch.complex64, device="cuda"))
+    for a in got:
+        root = a
+        while isinstance(root.base, np.ndarray):
+            root = root.base
+        held = root.base.untyped_storage().nbytes() if isinstance(root.base, torch.Tensor) else root.nbytes
+        assert held == a.nbytes
+    assert not np.shares_memory(*got)
