@@ -316,7 +316,7 @@ struct Segment {
 struct GraphKey {
   void* ws;
   int dev, group, n_ticks;
-  std::vector<int> shape;  // flattened segments
+  std::vector<int> shape;  // flattened lines of segments
   bool operator<(const GraphKey& o) const {
     return std::tie(ws, dev, group, n_ticks, shape) <
            std::tie(o.ws, o.dev, o.group, o.n_ticks, o.shape);
@@ -406,28 +406,43 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
   return SP_OK;
 }
 
-// Every segment of a group.  The sizes whose passes take more than one round of
-// the SMs share one line of launches; a size that leaves SMs idle gets its own,
-// on an auxiliary stream forked from `st` and joined back into it (in a capture
-// this forms parallel graph branches), unless it nearly fills them and is a
-// small part of the work.  Lines that all fill the chip get in one another's
-// way: waiting CTAs of one hold SMs that another could use.  us per iteration
-// with a line per size / as here: 64 x 256^2 + 32 x 512^2 + 8 x 1024^2 + 2 x 2048^2
-// 460 / 402; 16 x 512^2 + 4 x 1024^2 136 / 118; 16 x 256^2 + 8 x 512^2 + 3 x 1024^2 +
-// 2048^2 245 / 201 alone, 219 / 176 with calls on three streams (the 256^2
-// trials in a line of their own: 187 and 210).  Everything in one line is slower
-// where sizes leave SMs idle (512^2 + 1024^2: 29 / 34).  Beyond kLineRounds
-// rounds in all, what the overlap saves at the ends of passes is small, and sizes
-// that run side by side use memory and issue slots more evenly, so each gets a
-// line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds 1775 / 1779,
-// 182 rounds (70 x 1024^2 + 35 x 2048^2) 3428 / 3483, 214 rounds 3840 / 3911.
-// The joins are made even after a failed launch, so a capture never ends with
-// unjoined work.
+// How a group's segments are launched: line[0] on the caller's stream, the others
+// beside it on auxiliary streams.
+struct Lines {
+  std::vector<std::vector<Segment>> line;
+  bool beside;  // the lines' passes know of one another (PassArgs.late, LINE kernels)
+};
+
+// The sizes whose passes take more than one round of the SMs share one line of
+// launches; a size that leaves SMs idle gets its own, unless it nearly fills them
+// and is a small part of the work.  Lines that all fill the chip get in one
+// another's way: waiting CTAs of one hold SMs that another could use.  us per
+// iteration with a line per size / as here: 64 x 256^2 + 32 x 512^2 + 8 x 1024^2 +
+// 2 x 2048^2 460 / 402; 16 x 512^2 + 4 x 1024^2 136 / 118; 16 x 256^2 + 8 x 512^2 +
+// 3 x 1024^2 + 2048^2 249 / 181.
+// A size of 3/4 to one round with less than a fifth of the work costs a lone call
+// up to 6% in the line and gains with calls on several streams, as a serving loop
+// has them.  In a line of its own / in the line, alone and with two calls at once:
+//   16 x 256^2 + 8 x 512^2 + 3 x 1024^2 + 2048^2  176 / 182, 200 / 189
+//   16 x 256^2 + 16 x 512^2 + 2 x 2048^2          217 / 224, 241 / 229
+//   4 x 512^2 + 4 x 1024^2 + 2048^2               164 / 164, 187 / 169
+//   1024^2 + 3 x 2048^2                           242 / 247, 244 / 237
+//   15 x 256^2 + 6 x 1024^2                        97 /  95, 106 /  92
+//   18 x 256^2 + 30 x 512^2                       102 / 107, 108 /  99
+//   20 x 512^2 + 1024^2                            88 /  82,  93 /  81
+//   14 x 256^2 + 2 x 2048^2                       160 / 170, 167 / 168
+// With a greater part of the work, or fewer rounds, the lone call loses more:
+//   60 x 256^2 + 4 x 512^2                         57 /  63,  67 /  58
+//   18 x 256^2 + 8 x 512^2                         41 /  47,  45 /  42
+//   12 x 256^2 + 20 x 512^2                        73 /  75,  76 /  70
+// Beyond kLineRounds rounds in all, what the overlap saves at the ends of passes is
+// small, and sizes that run side by side use memory and issue slots more evenly, so
+// each gets a line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds
+// 1775 / 1779, 182 rounds (70 x 1024^2 + 35 x 2048^2) 3428 / 3483, 214 rounds
+// 3840 / 3911.
 constexpr double kLineRounds = 90;
-static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, const Item* items,
-                        const int2* jobs, const float2* tw, ForkPool* P, cudaStream_t st) {
-  if (P == nullptr || segs.size() == 1)
-    return launch_line(segs, slots, items, jobs, tw, false, st);
+static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
+  if (!concurrent || segs.size() == 1) return {{segs}, false};
   double work = 0, rounds = 0;
   for (const Segment& sg : segs) {
     work += sg.work;
@@ -437,15 +452,25 @@ static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, con
   auto shared = [&](const Segment& sg) {
     return !apart && (sg.rounds > 1.0 || (sg.rounds > 0.75 && sg.work < 0.2 * work));
   };
-  std::vector<std::vector<Segment>> lines(1);  // [0] on `st`
+  Lines r{std::vector<std::vector<Segment>>(1), false};
   for (const Segment& sg : segs)
-    if (shared(sg)) lines[0].push_back(sg);
+    if (shared(sg)) r.line[0].push_back(sg);
   for (const Segment& sg : segs) {
     if (shared(sg)) continue;
-    if (lines[0].empty()) lines[0].push_back(sg);
-    else lines.push_back({sg});
+    if (r.line[0].empty()) r.line[0].push_back(sg);
+    else r.line.push_back({sg});
   }
-  const int n_aux = (int)lines.size() - 1;
+  r.beside = r.line.size() > 1 && !apart;
+  return r;
+}
+
+// Launch a group's lines, the auxiliary streams forked from `st` and joined back
+// into it (in a capture this forms parallel graph branches).  The joins are made
+// even after a failed launch, so a capture never ends with unjoined work.
+static int launch_ticks(const Lines& lines, const Slot* slots, const Item* items, const int2* jobs,
+                        const float2* tw, ForkPool* P, cudaStream_t st) {
+  const int n_aux = (int)lines.line.size() - 1;
+  if (n_aux == 0) return launch_line(lines.line[0], slots, items, jobs, tw, lines.beside, st);
   SP_CUDA_TRY(cudaEventRecord(P->events[0], st));
   int rc = SP_OK;
   int forked = 0;
@@ -456,9 +481,10 @@ static int launch_ticks(const std::vector<Segment>& segs, const Slot* slots, con
       break;
     }
     forked = i + 1;
-    if (rc == SP_OK) rc = launch_line(lines[i + 1], slots, items, jobs, tw, !apart, P->streams[i]);
+    if (rc == SP_OK)
+      rc = launch_line(lines.line[i + 1], slots, items, jobs, tw, lines.beside, P->streams[i]);
   }
-  if (rc == SP_OK) rc = launch_line(lines[0], slots, items, jobs, tw, n_aux > 0 && !apart, st);
+  if (rc == SP_OK) rc = launch_line(lines.line[0], slots, items, jobs, tw, lines.beside, st);
   for (int i = 0; i < forked; ++i) {
     const cudaError_t e1 = cudaEventRecord(P->events[1 + i], P->streams[i]);
     const cudaError_t e2 = cudaStreamWaitEvent(st, P->events[1 + i], 0);
@@ -672,16 +698,23 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
   if (concurrent && max_segs > 1) SP_CUDA_TRY(fork_pool(dev, (int)max_segs - 1, &pool));
 
   for (int g = 0; g < n_groups; ++g) {
+    const Lines lines = lines_of(segs[g], concurrent);
     if (!use_graph) {
-      const int rc = launch_ticks(segs[g], dslots, ditems, djobs, tw, pool, st);
+      const int rc = launch_ticks(lines, dslots, ditems, djobs, tw, pool, st);
       if (rc != SP_OK) return rc;
       continue;
     }
     GraphKey key{workspace_dev, dev, g, ticks[g], {}};
-    for (const Segment& sg : segs[g])
-      key.shape.insert(key.shape.end(), {sg.N, sg.E, sg.first, sg.count, sg.grid[0], sg.grid[1], sg.kind[0], sg.kind[1],
-                                         sg.pc_first, sg.pc_count, sg.pc_grid, sg.pc_egrid,
-                                         std::min(sg.ticks, sg.col_ticks), sg.pc_mask, sg.ticks});
+    // (by lines: how they are split also depends on the algorithms)
+    key.shape.push_back(lines.beside);
+    for (const auto& line : lines.line) {
+      key.shape.push_back((int)line.size());
+      for (const Segment& sg : line)
+        key.shape.insert(key.shape.end(), {sg.N, sg.E, sg.first, sg.count, sg.grid[0], sg.grid[1],
+                                           sg.kind[0], sg.kind[1], sg.pc_first, sg.pc_count, sg.pc_grid,
+                                           sg.pc_egrid, std::min(sg.ticks, sg.col_ticks), sg.pc_mask,
+                                           sg.ticks});
+    }
     cudaGraphExec_t exec = nullptr;
     {
       std::lock_guard<std::mutex> lock(g_graph_mutex);
@@ -691,7 +724,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
     if (!exec) {
       cudaGraph_t graph = nullptr;
       SP_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      const int rc = launch_ticks(segs[g], dslots, ditems, djobs, tw, pool, st);
+      const int rc = launch_ticks(lines, dslots, ditems, djobs, tw, pool, st);
       const cudaError_t ce = cudaStreamEndCapture(st, &graph);
       if (rc != SP_OK) {
         if (graph) cudaGraphDestroy(graph);

@@ -108,3 +108,35 @@ def test_early_passes_read_what_the_last_tick_wrote(mix):
     for k, (a, b) in enumerate(zip(mixed, alone)):
         assert torch.equal(torch.view_as_real(a), torch.view_as_real(b)), k
     eng.close()
+
+
+def test_graphs_of_different_lines_are_kept_apart():
+    """16 x 256^2 share the other sizes' line while they are less than a fifth of the
+    work, and get their own once they run DM (twice the work): a batch of the same
+    shape in the same workspace must not replay the other's graph."""
+    import torch
+    from als_speckle_b200 import _lib
+    from als_speckle_b200.engine import Engine, TrialSpec
+    mix = ((256, 16), (512, 9), (1024, 2))
+
+    def specs(alg):
+        out = []
+        for N, count in mix:
+            M = torch.ones((N, N), device="cuda")
+            a = alg if N == 256 else "hio"
+            out += [TrialSpec(psi=torch.zeros((N, N), dtype=torch.complex64, device="cuda"), modulus=M,
+                              support=M, iterations=3, order=((a, 3),), beta=0.9, random_phase=True,
+                              seed=2, trial=k) for k in range(count)]
+        return out
+
+    eng = Engine(use_graph=True)
+    stream = torch.cuda.Stream()
+    counts = [_lib.lib.sp_engine_graph_count()]
+    for alg in ("dm", "hio", "dm", "raar"):  # DM first: its workspace is the larger one
+        sp = specs(alg)
+        stream.wait_stream(torch.cuda.current_stream())
+        eng.solve(sp, stream=stream)
+        stream.synchronize()
+        counts.append(_lib.lib.sp_engine_graph_count())
+    assert [c - counts[0] for c in counts] == [0, 1, 2, 2, 2]
+    eng.close()
