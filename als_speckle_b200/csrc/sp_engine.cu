@@ -584,9 +584,12 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
         else if (trials[i].init == SP_INIT_RANDOM_PHASE) sg.col_ticks = std::max(sg.col_ticks, 1);
       }
       for (int p = 0; p < 2; ++p) {
-        if (use_small_ctas(N, E, count, sms)) sg.kind[p] = p == 0 ? kPassColSmall : kPassRowSmall;
+        const bool small = use_small_ctas(N, E, count, sms);
+        if (small) sg.kind[p] = p == 0 ? kPassColSmall : kPassRowSmall;
         int per_sm = occ[sg.kind[p]];
-        if (opts && opts->ctas_per_sm > 0) per_sm = std::min(per_sm, (int)opts->ctas_per_sm);
+        // (the cap is in large CTAs)
+        if (opts && opts->ctas_per_sm > 0)
+          per_sm = (int)std::min<int64_t>(per_sm, (int64_t)opts->ctas_per_sm * (small ? kThreads / kSmallThreads : 1));
         const int units = count * pass_units(N, E, sg.kind[p]);
         sg.grid[p] = std::max(1, std::min(units, sms * per_sm));
         sg.rounds = (double)units / (sms * per_sm);  // (of the row pass, the last)

@@ -93,7 +93,8 @@ typedef struct sp_run_opts {
   int32_t use_graph;       /* capture each group's launch sequence in a CUDA graph
                               (needs a non-default stream; graphs are cached per
                               workspace and launch shape) */
-  int32_t ctas_per_sm;     /* cap on resident CTAs per SM of the persistent grid (0 = max) */
+  int32_t ctas_per_sm;     /* cap on resident CTAs per SM of the persistent grid (0 = max);
+                              four of the 64-thread CTAs of small calls count as one */
   int32_t e_per_logn[13];  /* values per thread (16 or 32) for N = 2^l; 0 = default */
 } sp_run_opts;
 
