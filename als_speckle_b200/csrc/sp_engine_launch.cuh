@@ -353,10 +353,11 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
 // CTAs, small CTAs in brackets: 256^2 x 1 8.5 / 6.1 [64], x 2 8.6 / 7.4 [128],
 // x 4 8.7 / 8.5 [256], x 8 9.3 / 10.5 [512]; 512^2 x 1 12.8 / 11.2 [128], x 4
 // 16.1 / 17.4 [512]; 128^2 x 1 14.7 / 8.4 [8], x 36 15.5 / 12.1 [288]; 64^2 x
-// 40 11.9 / 9.4 [80].  At 1024^2 a trial is 128 items already.
+// 40 11.9 / 9.4 [80].  At 1024^2 a trial is 128 items already, and at 512^2 with
+// E < 32 one trial is more small CTAs than the rule takes.
 constexpr int kSmallThreads = 64;
 __host__ __device__ constexpr bool has_small_ctas(int N, int E) {
-  return N >= 64 && N <= 512 && pass_split(N, E, kSmallThreads) > 1;
+  return N >= 64 && (N < 512 || (N == 512 && E == 32)) && pass_split(N, E, kSmallThreads) > 1;
 }
 
 // pass kinds: 0 column, 1 row, the same in small CTAs, and the same (large) for
