@@ -345,8 +345,8 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
 
 // Lone trials and small batches: when the items of kThreads-thread CTAs are
 // too few for the chip (a 256^2 trial is 16 of them at E = 16, on 16 of 148
-// SMs), both passes run in kSmallThreads-thread CTAs on quarter items instead
-// (the same kernels, so bitwise the same results): a lone pass is bound by its
+// SMs), both passes run in kSmallThreads-thread CTAs on quarter items (half items at
+// 64^2 with E = 32) instead (the same kernels, so bitwise the same results): a lone pass is bound by its
 // warps' own instruction chains, which run faster with 2 warps on an SM than
 // with 8.  Taken up to two small CTAs per SM (one at 512^2, where two of them
 // are as slow as a large one); measured, us per iteration in large / small

@@ -83,7 +83,9 @@ __global__ void __launch_bounds__(256) blur_kernel(const void* __restrict__ in,
 
 // ---------------------------------------------------------------------------
 // connected parts of a mask: 8 neighbours, periodic.  Union-find over pixel
-// indexes, always towards the smaller one, so a part's root is its first pixel
+// indexes by atomic minima (Playne & Hawick, IEEE Trans. Parallel Distrib. Syst.
+// 29, 2018) with path halving (Tarjan & van Leeuwen, J. ACM 31, 1984), always
+// towards the smaller index, so a part's root is its first pixel
 // in raster order (the order in which the reference finds the parts).  Runs
 // inside a warp's 32 pixels start out linked to their first pixel; then every
 // pixel joins its neighbours to the left (across warps) and above where the

@@ -78,7 +78,8 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return r;
 }
 
-// row pairs of a warp for MQ column groups: 48-64 accumulator registers
+// row pairs of a warp for MQ column groups, four accumulator registers each: 16 to
+// 64 for up to four groups, 40 to 64 for more
 __host__ __device__ constexpr int reg_pairs(int MQ) { return MQ <= 4 ? 4 : 2; }
 __host__ __device__ constexpr int reg_tile_rows(int MQ) { return kRegWarps * 2 * reg_pairs(MQ); }
 

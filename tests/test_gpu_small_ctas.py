@@ -45,3 +45,12 @@ def test_small_ctas_match_large(N, E, counts, alg):
             # FP64 sums of the same FP32 partials, added in any order
             np.testing.assert_allclose(err[k], large[2][k], rtol=1e-12)
     eng.close()
+
+
+@pytest.mark.parametrize("alg", ["hio", "dm"])
+@pytest.mark.parametrize("N,E,counts", [
+    # the other pairs that have both; small CTAs of a trial: (64, 8) and (64, 16)
+    # 8 and 4, the other two 32; at (64, 32) above an item is two, not four
+    (64, 8, (1, 37, 38)), (64, 16, (1, 74, 75)), (128, 8, (1, 9, 10)), (256, 32, (1, 9, 10))])
+def test_small_ctas_match_large_for_every_e(N, E, counts, alg):
+    test_small_ctas_match_large(N, E, counts, alg)
