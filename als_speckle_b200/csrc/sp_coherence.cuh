@@ -110,8 +110,14 @@ __global__ void __launch_bounds__(kThreads, 4) pc_cols_a_kernel(PcArgs a) {
 }
 
 // W: W = IFFT_rows(FFT_rows(W) * ipsf), unnormalised.
+// CTAs per SM it is compiled for: four at 512^2, where they fit 64 registers
+// without a spill; below, 64 registers spill 100 bytes and two CTAs without spills
+// are faster (six iterations of 256^2 with an ipsf, 64 / 80 / 128 registers: 3
+// trials 147 / 146 / 141 us, 8 179 / 177 / 173, 14 216 / 213 / 209, 50 532 / 539 /
+// 535; 4 of 64^2 157 / 153 / 151).
+__host__ __device__ constexpr int pc_w_ctas(int N) { return N < 512 ? 2 : (N == 512 ? 4 : 3); }
 template <int N>
-__global__ void __launch_bounds__(kThreads, N <= 512 ? 4 : 3) pc_rows_w_kernel(PcArgs a) {
+__global__ void __launch_bounds__(kThreads, pc_w_ctas(N)) pc_rows_w_kernel(PcArgs a) {
   constexpr int E = pc_e(N), T = N / E, L = lines_per_item(N, E), SH = pad_shift(E);
   using Sync = typename std::conditional<(T <= 32), WarpSync, BlockSync>::type;
   extern __shared__ float2 smem[];

@@ -42,3 +42,11 @@ def test_batches_match_alone(N, counts, mode, alg):
             if k < c:
                 np.testing.assert_array_equal(batch[k], alone[k])
     eng.close()
+
+
+@pytest.mark.parametrize("mode", ["ipsf", "both"])
+@pytest.mark.parametrize("N,counts", [(64, (75, 149)), (128, (19, 38)), (256, (6, 19))])
+def test_batches_match_alone_at_small_n(N, counts, mode):
+    """Counts of one to a few CTAs per SM at the sizes whose row kernel is compiled
+    for two CTAs on an SM."""
+    test_batches_match_alone(N, counts, mode, "hio")
