@@ -407,7 +407,7 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
 }
 
 // How a group's segments are launched: line[0] on the caller's stream, the others
-// beside it on auxiliary streams.
+// beside it on auxiliary streams, or after it where there are none.
 struct Lines {
   std::vector<std::vector<Segment>> line;
   bool beside;  // the lines' passes know of one another (PassArgs.late, LINE kernels)
@@ -440,9 +440,14 @@ struct Lines {
 // each gets a line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds
 // 1775 / 1779, 182 rounds (70 x 1024^2 + 35 x 2048^2) 3428 / 3483, 214 rounds
 // 3840 / 3911.
+// Without auxiliary streams (`concurrent` false) the lines follow one another, and
+// only sizes of more than one round share one: what the others leave idle, a pass
+// of one of them cannot use.  20 iterations, all in one line / as here:
+// 16 x 256^2 + 4 x 512^2 742 / 634; 4 x 512^2 + 1024^2 829 / 699; 12 x 256^2 +
+// 2 x 1024^2 983 / 903; 30 x 256^2 + 5 x 512^2 893 / 897.
 constexpr double kLineRounds = 90;
 static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
-  if (!concurrent || segs.size() == 1) return {{segs}, false};
+  if (segs.size() == 1) return {{segs}, false};
   double work = 0, rounds = 0;
   for (const Segment& sg : segs) {
     work += sg.work;
@@ -450,7 +455,7 @@ static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
   }
   const bool apart = rounds > kLineRounds;
   auto shared = [&](const Segment& sg) {
-    return !apart && (sg.rounds > 1.0 || (sg.rounds > 0.75 && sg.work < 0.2 * work));
+    return !apart && (sg.rounds > 1.0 || (concurrent && sg.rounds > 0.75 && sg.work < 0.2 * work));
   };
   Lines r{std::vector<std::vector<Segment>>(1), false};
   for (const Segment& sg : segs)
@@ -460,17 +465,23 @@ static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
     if (r.line[0].empty()) r.line[0].push_back(sg);
     else r.line.push_back({sg});
   }
-  r.beside = r.line.size() > 1 && !apart;
+  r.beside = concurrent && r.line.size() > 1 && !apart;
   return r;
 }
 
-// Launch a group's lines, the auxiliary streams forked from `st` and joined back
+// Launch a group's lines, the auxiliary streams (of `P`, if any) forked from `st` and joined back
 // into it (in a capture this forms parallel graph branches).  The joins are made
 // even after a failed launch, so a capture never ends with unjoined work.
 static int launch_ticks(const Lines& lines, const Slot* slots, const Item* items, const int2* jobs,
                         const float2* tw, ForkPool* P, cudaStream_t st) {
   const int n_aux = (int)lines.line.size() - 1;
-  if (n_aux == 0) return launch_line(lines.line[0], slots, items, jobs, tw, lines.beside, st);
+  if (P == nullptr || n_aux == 0) {
+    for (const auto& line : lines.line) {
+      const int rc = launch_line(line, slots, items, jobs, tw, lines.beside, st);
+      if (rc != SP_OK) return rc;
+    }
+    return SP_OK;
+  }
   SP_CUDA_TRY(cudaEventRecord(P->events[0], st));
   int rc = SP_OK;
   int forked = 0;
