@@ -425,9 +425,10 @@ size_t pc_smem_bytes(int per_sm) {
 }
 
 // which: 0 = A, 1 = W, 2 = B1, 3 = R, 4 = B.  R keeps a plain launch: it lives on
-// L1 hits, which padding would cost.
+// L1 hits, which padding would cost.  `pad_sms`: SMs of the device where the jobs'
+// size has them to itself, else 0: padded CTAs would shut other sizes' passes out.
 template <int N>
-cudaError_t launch_pc_t(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) {
+cudaError_t launch_pc_t(int which, int grid, int pad_sms, cudaStream_t st, const PcArgs& a) {
   if (which == 3) {
     pc_rescale_kernel<N><<<grid, kThreads, 0, st>>>(a);
     return cudaGetLastError();
@@ -437,7 +438,8 @@ cudaError_t launch_pc_t(int which, int grid, int n_sms, cudaStream_t st, const P
                       : which == 2 ? pc_cols_b1_kernel<N>
                                    : pc_cols_b_kernel<N>;
   if constexpr (pc_programmatic(N))
-    return launch_pdl(k, grid, kThreads, pc_smem_bytes<N>((grid + n_sms - 1) / n_sms), st, a);
+    if (pad_sms > 0)
+      return launch_pdl(k, grid, kThreads, pc_smem_bytes<N>((grid + pad_sms - 1) / pad_sms), st, a);
   k<<<grid, kThreads, pc_smem_bytes<N>(4), st>>>(a);
   return cudaGetLastError();
 }
@@ -462,7 +464,7 @@ constexpr int pc_items_per_job() { return N / lines_per_item(N, pc_e(N)); }
 
 namespace sp {
 #define SP_DECLARE_PC(N)                                                              \
-  cudaError_t launch_pc_n##N(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a); \
+  cudaError_t launch_pc_n##N(int which, int grid, int pad_sms, cudaStream_t st, const PcArgs& a); \
   cudaError_t pc_setup_n##N();
 SP_DECLARE_PC(8)
 SP_DECLARE_PC(16)
@@ -476,8 +478,8 @@ SP_DECLARE_PC(2048)
 SP_DECLARE_PC(4096)
 
 #define SP_DEFINE_PC(N)                                                                \
-  cudaError_t launch_pc_n##N(int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) { \
-    return launch_pc_t<N>(which, grid, n_sms, st, a);                                        \
+  cudaError_t launch_pc_n##N(int which, int grid, int pad_sms, cudaStream_t st, const PcArgs& a) { \
+    return launch_pc_t<N>(which, grid, pad_sms, st, a);                                        \
   }                                                                                    \
   cudaError_t pc_setup_n##N() { return pc_setup_t<N>(); }
 }  // namespace sp

@@ -53,18 +53,18 @@ static cudaError_t pass_setup(int N, int E, int* occ) {
   }
 }
 
-static cudaError_t launch_pc(int N, int which, int grid, int n_sms, cudaStream_t st, const PcArgs& a) {
+static cudaError_t launch_pc(int N, int which, int grid, int pad_sms, cudaStream_t st, const PcArgs& a) {
   switch (N) {
-    case 8: return launch_pc_n8(which, grid, n_sms, st, a);
-    case 16: return launch_pc_n16(which, grid, n_sms, st, a);
-    case 32: return launch_pc_n32(which, grid, n_sms, st, a);
-    case 64: return launch_pc_n64(which, grid, n_sms, st, a);
-    case 128: return launch_pc_n128(which, grid, n_sms, st, a);
-    case 256: return launch_pc_n256(which, grid, n_sms, st, a);
-    case 512: return launch_pc_n512(which, grid, n_sms, st, a);
-    case 1024: return launch_pc_n1024(which, grid, n_sms, st, a);
-    case 2048: return launch_pc_n2048(which, grid, n_sms, st, a);
-    case 4096: return launch_pc_n4096(which, grid, n_sms, st, a);
+    case 8: return launch_pc_n8(which, grid, pad_sms, st, a);
+    case 16: return launch_pc_n16(which, grid, pad_sms, st, a);
+    case 32: return launch_pc_n32(which, grid, pad_sms, st, a);
+    case 64: return launch_pc_n64(which, grid, pad_sms, st, a);
+    case 128: return launch_pc_n128(which, grid, pad_sms, st, a);
+    case 256: return launch_pc_n256(which, grid, pad_sms, st, a);
+    case 512: return launch_pc_n512(which, grid, pad_sms, st, a);
+    case 1024: return launch_pc_n1024(which, grid, pad_sms, st, a);
+    case 2048: return launch_pc_n2048(which, grid, pad_sms, st, a);
+    case 4096: return launch_pc_n4096(which, grid, pad_sms, st, a);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -307,7 +307,7 @@ struct Segment {
   int pc_egrid;                     // grid of the tiled rescale kernel
   int col_ticks;                    // the column pass runs at ticks [0, col_ticks)
   int pc_mask;                      // partial-coherence kernels launched (bit = which)
-  int sms;                          // of the device
+  int pc_pad_sms;                   // SMs, where no other size runs beside its jobs; else 0 (launch_pc_t)
   double rounds;                    // of the SMs that a row pass takes
   double work;                      // pixels times projections of a tick
   int ticks;                        // ticks of this segment's longest trial (n_iter + 1)
@@ -386,7 +386,7 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
             PcArgs pa{slots, jobs + sg.pc_first, sg.pc_count, k, tw};
             for (int w = 0; w < 5; ++w)
               if (sg.pc_mask & (1 << w))
-                SP_CUDA_TRY(launch_pc(sg.N, w, w == 3 ? sg.pc_egrid : sg.pc_grid, sg.sms, st, pa));
+                SP_CUDA_TRY(launch_pc(sg.N, w, w == 3 ? sg.pc_egrid : sg.pc_grid, sg.pc_pad_sms, st, pa));
             prev = i;
           }
           if (k >= sg.col_ticks) continue;  // no column work left in this segment
@@ -421,25 +421,25 @@ struct Lines {
 // 2 x 2048^2 460 / 402; 16 x 512^2 + 4 x 1024^2 136 / 118; 16 x 256^2 + 8 x 512^2 +
 // 3 x 1024^2 + 2048^2 249 / 181.
 // A size of 3/4 to one round with less than a fifth of the work costs a lone call
-// up to 6% in the line and gains with calls on several streams, as a serving loop
+// up to 4% in the line and gains with calls on several streams, as a serving loop
 // has them.  In a line of its own / in the line, alone and with two calls at once:
 //   16 x 256^2 + 8 x 512^2 + 3 x 1024^2 + 2048^2  176 / 182, 200 / 189
 //   16 x 256^2 + 16 x 512^2 + 2 x 2048^2          217 / 224, 241 / 229
 //   4 x 512^2 + 4 x 1024^2 + 2048^2               164 / 164, 187 / 169
 //   1024^2 + 3 x 2048^2                           242 / 247, 244 / 237
-//   15 x 256^2 + 6 x 1024^2                        97 /  95, 106 /  92
-//   18 x 256^2 + 30 x 512^2                       102 / 107, 108 /  99
 //   20 x 512^2 + 1024^2                            88 /  82,  93 /  81
-//   14 x 256^2 + 2 x 2048^2                       160 / 170, 167 / 168
 // With a greater part of the work, or fewer rounds, the lone call loses more:
 //   60 x 256^2 + 4 x 512^2                         57 /  63,  67 /  58
-//   18 x 256^2 + 8 x 512^2                         41 /  47,  45 /  42
 //   12 x 256^2 + 20 x 512^2                        73 /  75,  76 /  70
 // Beyond kLineRounds rounds in all, what the overlap saves at the ends of passes is
 // small, and sizes that run side by side use memory and issue slots more evenly, so
 // each gets a line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds
 // 1775 / 1779, 182 rounds (70 x 1024^2 + 35 x 2048^2) 3428 / 3483, 214 rounds
 // 3840 / 3911.
+// A partially coherent size gets a line of its own: its five kernels, which start
+// when all before them is complete, would hold up every other size of a line (18 x
+// 512^2 and 4 x 1024^2 with an ipsf + 26 x 256^2, 19, 11 and 7 iterations: 4.09 ms
+// in the line, 3.79 as here).
 // Without auxiliary streams (`concurrent` false) the lines follow one another, and
 // only sizes of more than one round share one: what the others leave idle, a pass
 // of one of them cannot use.  20 iterations, all in one line / as here:
@@ -455,7 +455,8 @@ static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
   }
   const bool apart = rounds > kLineRounds;
   auto shared = [&](const Segment& sg) {
-    return !apart && (sg.rounds > 1.0 || (concurrent && sg.rounds > 0.75 && sg.work < 0.2 * work));
+    return !apart && sg.pc_count == 0 &&
+           (sg.rounds > 1.0 || (concurrent && sg.rounds > 0.75 && sg.work < 0.2 * work));
   };
   Lines r{std::vector<std::vector<Segment>>(1), false};
   for (const Segment& sg : segs)
@@ -568,6 +569,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
   hj.reserve(L.n_jobs);
   std::vector<std::vector<Segment>> segs(n_groups);
   std::vector<int> ticks(n_groups, 0);
+  int sms = 1;
   for (int g = 0; g < n_groups; ++g) {
     for (int N = kMinN; N <= kMaxN; N *= 2) {
       const int E = chosen_e(N, opts);
@@ -579,9 +581,9 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       }
       const int count = (int)hi.size() - first;
       if (count == 0) continue;
-      int occ[kPassKinds], sms = 1;
+      int occ[kPassKinds];
       SP_CUDA_TRY(occupancy_for(N, E, occ, &sms));
-      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, sms, 1.0, 0.0, 0};
+      Segment sg{N, E, first, count, {1, 1}, {kPassCol, kPassRow}, (int)hj.size(), 0, 1, 1, 0, 0, 0, 1.0, 0.0, 0};
       for (int i = gstart[g]; i < gstart[g + 1]; ++i)
         if (trials[i].n == N) sg.work += (double)N * N * (uses_dm(trials[i]) ? 2 : 1);
       for (int i = gstart[g]; i < gstart[g + 1]; ++i)
@@ -620,15 +622,18 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
       if (sg.pc_count > 0) {
         SP_CUDA_TRY(pc_ready(N));
         const int per_job = N / lines_per_item(N, pc_e(N));
-        // up to 512^2 a CTA for every item (the hardware deals the uneven last
-        // round out: 2-5% on 16-45 trials); above, persistent CTAs, whose
-        // larger twiddle tables are worth keeping
-        const int64_t units = (int64_t)sg.pc_count * per_job;
-        sg.pc_grid = (int)std::max<int64_t>(1, N <= 512 ? units : std::min<int64_t>(units, sms * 4));
+        sg.pc_grid = (int)std::min<int64_t>((int64_t)sg.pc_count * per_job, INT32_MAX);
         const int64_t tiles = (int64_t)sg.pc_count * N * N / rescale_tile_pixels(N);
         sg.pc_egrid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)sms * 8));
       }
       segs[g].push_back(sg);
+    }
+    for (Segment& sg : segs[g]) {
+      // Alone and up to 512^2 a CTA for every item (the hardware deals the uneven
+      // last round out: 2-5% on 16-45 trials); else persistent CTAs, whose larger
+      // twiddle tables are worth keeping.
+      sg.pc_pad_sms = segs[g].size() == 1 && sg.N <= 512 ? sms : 0;
+      if (sg.pc_pad_sms == 0) sg.pc_grid = std::min(sg.pc_grid, sms * 4);
     }
     for (int i = gstart[g]; i < gstart[g + 1]; ++i) {
       const sp_trial& t = trials[i];
