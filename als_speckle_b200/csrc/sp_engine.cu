@@ -440,20 +440,24 @@ struct Lines {
 // when all before them is complete, would hold up every other size of a line (18 x
 // 512^2 and 4 x 1024^2 with an ipsf + 26 x 256^2, 19, 11 and 7 iterations: 4.09 ms
 // in the line, 3.79 as here).
+// A caller's cap on resident CTAs (`capped`) leaves an SM's room to whatever else
+// runs there: passes in a shared line would start in that room at once, so each
+// size gets its own line then too (one CTA per SM, 32 x 256^2 DM + 13 x 512^2 +
+// 2048^2: 1857 us in the line, 1799 apart).
 // Without auxiliary streams (`concurrent` false) the lines follow one another, and
 // only sizes of more than one round share one: what the others leave idle, a pass
 // of one of them cannot use.  20 iterations, all in one line / as here:
 // 16 x 256^2 + 4 x 512^2 742 / 634; 4 x 512^2 + 1024^2 829 / 699; 12 x 256^2 +
 // 2 x 1024^2 983 / 903; 30 x 256^2 + 5 x 512^2 893 / 897.
 constexpr double kLineRounds = 90;
-static Lines lines_of(const std::vector<Segment>& segs, bool concurrent) {
+static Lines lines_of(const std::vector<Segment>& segs, bool concurrent, bool capped) {
   if (segs.size() == 1) return {{segs}, false};
   double work = 0, rounds = 0;
   for (const Segment& sg : segs) {
     work += sg.work;
     rounds += sg.rounds;
   }
-  const bool apart = rounds > kLineRounds;
+  const bool apart = capped || rounds > kLineRounds;
   auto shared = [&](const Segment& sg) {
     return !apart && sg.pc_count == 0 &&
            (sg.rounds > 1.0 || (concurrent && sg.rounds > 0.75 && sg.work < 0.2 * work));
@@ -717,7 +721,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
   if (concurrent && max_segs > 1) SP_CUDA_TRY(fork_pool(dev, (int)max_segs - 1, &pool));
 
   for (int g = 0; g < n_groups; ++g) {
-    const Lines lines = lines_of(segs[g], concurrent);
+    const Lines lines = lines_of(segs[g], concurrent, opts && opts->ctas_per_sm > 0);
     if (!use_graph) {
       const int rc = launch_ticks(lines, dslots, ditems, djobs, tw, pool, st);
       if (rc != SP_OK) return rc;

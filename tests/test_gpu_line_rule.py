@@ -78,3 +78,8 @@ def test_partially_coherent_sizes_run_beside_the_line(mix, ipsf, lines, tmp_path
         shared = [{e["args"]["shared memory"] for e in ks if name in e["name"]} for ks in (kernels, alone)]
         assert len(shared[0]) == 1 and max(shared[0]) < 64 * 1024
         assert max(shared[0]) <= min(shared[1])
+
+
+@pytest.mark.parametrize("mix", [((512, 10), (1024, 3)), ((256, 20), (512, 10), (1024, 3))])
+def test_capped_sizes_run_side_by_side(mix, tmp_path):
+    _check(mix, [{N} for N, _ in mix], tmp_path, ctas_per_sm=1)
