@@ -431,6 +431,19 @@ struct Lines {
 // With a greater part of the work, or fewer rounds, the lone call loses more:
 //   60 x 256^2 + 4 x 512^2                         57 /  63,  67 /  58
 //   12 x 256^2 + 20 x 512^2                        73 /  75,  76 /  70
+// Two sizes share a line only if both are 512^2 or more and one is larger: a pass
+// of a smaller size leaves room on its SMs for the other's, and two of them run
+// better side by side; from three sizes on, one of them above 512^2, a line is
+// better whatever they are.  10 iterations, side by side / in the line:
+//   19 x 256^2 + 5 x 512^2             383 / 472     30 x 256^2 + 9 x 512^2  566 / 580
+//   37 x 256^2 + 18 x 512^2            885 / 884     19 x 256^2 + 3 x 1024^2 630 / 692
+//   30 x 256^2 + 2048^2               1134 / 1210    37 x 256^2 + 3 x 1024^2 795 / 773
+//   100 x 128^2 + 20 x 256^2 + 6 x 512^2 811 / 860   100 x 128^2 + 6 x 512^2 597 / 641
+//   5 x 512^2 + 2 x 1024^2             598 / 568     18 x 512^2 + 4 x 1024^2 1304 / 1132
+//   3 x 1024^2 + 2048^2               1499 / 1320    10 x 512^2 + 2048^2    1308 / 1265
+//   19 x 256^2 + 5 x 512^2 + 2 x 1024^2 844 / 795    80 x 128^2 + 20 x 256^2 + 3 x 1024^2
+//   1098 / 1014
+// (With two calls at once 18 x 512^2 + 4 x 1024^2 lose in the line, 1415 / 1500.)
 // Beyond kLineRounds rounds in all, what the overlap saves at the ends of passes is
 // small, and sizes that run side by side use memory and issue slots more evenly, so
 // each gets a line (and the plain kernels) again: 47 rounds 949 / 926, 95 rounds
@@ -458,15 +471,23 @@ static Lines lines_of(const std::vector<Segment>& segs, bool concurrent, bool ca
     rounds += sg.rounds;
   }
   const bool apart = capped || rounds > kLineRounds;
-  auto shared = [&](const Segment& sg) {
+  auto fits = [&](const Segment& sg) {
     return !apart && sg.pc_count == 0 &&
            (sg.rounds > 1.0 || (concurrent && sg.rounds > 0.75 && sg.work < 0.2 * work));
   };
+  int n = 0, small = 0, large = 0;
+  for (const Segment& sg : segs) {
+    if (!fits(sg)) continue;
+    ++n;
+    small += sg.N < 512;
+    large += sg.N > 512;
+  }
+  const bool share = !concurrent || (large > 0 && (n > 2 || small == 0));
   Lines r{std::vector<std::vector<Segment>>(1), false};
   for (const Segment& sg : segs)
-    if (shared(sg)) r.line[0].push_back(sg);
+    if (share && fits(sg)) r.line[0].push_back(sg);
   for (const Segment& sg : segs) {
-    if (shared(sg)) continue;
+    if (share && fits(sg)) continue;
     if (r.line[0].empty()) r.line[0].push_back(sg);
     else r.line.push_back({sg});
   }

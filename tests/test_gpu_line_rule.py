@@ -83,3 +83,13 @@ def test_partially_coherent_sizes_run_beside_the_line(mix, ipsf, lines, tmp_path
 @pytest.mark.parametrize("mix", [((512, 10), (1024, 3)), ((256, 20), (512, 10), (1024, 3))])
 def test_capped_sizes_run_side_by_side(mix, tmp_path):
     _check(mix, [{N} for N, _ in mix], tmp_path, ctas_per_sm=1)
+
+
+@pytest.mark.parametrize("mix,lines", [
+    (((256, 19), (512, 5)), [{256}, {512}]), (((256, 37), (1024, 3)), [{256}, {1024}]),
+    (((512, 5), (1024, 2)), [{512, 1024}]), (((1024, 2), (2048, 1)), [{1024, 2048}]),
+    (((256, 19), (512, 5), (1024, 2)), [{256, 512, 1024}]),
+    (((128, 100), (256, 20), (512, 6)), [{128}, {256}, {512}]),
+    (((128, 4), (512, 5), (1024, 2)), [{128}, {512, 1024}])])
+def test_sizes_of_a_pair_share_a_line_when_they_fill_their_sms(mix, lines, tmp_path):
+    _check(mix, lines, tmp_path)
