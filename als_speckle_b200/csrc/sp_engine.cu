@@ -369,9 +369,10 @@ static cudaError_t fork_pool(int dev, int branches, ForkPool** out) {
 // no data (their trials, planes and items are disjoint; slots, items and
 // transposed moduli are only read), so a pass that follows one of another size
 // starts on the SMs that one's last round leaves idle (PassArgs.overlap).
-// `beside`: other lines run concurrently (PassArgs.late).
+// `beside`: other lines run concurrently (PassArgs.late, or PassArgs.early where
+// `idle`).
 static int launch_line(const std::vector<Segment>& segs, const Slot* slots, const Item* items,
-                       const int2* jobs, const float2* tw, bool beside, cudaStream_t st) {
+                       const int2* jobs, const float2* tw, bool beside, bool idle, cudaStream_t st) {
   int ticks = 0;
   for (const Segment& sg : segs) ticks = std::max(ticks, sg.ticks);
   int prev = -1;  // segment of the previous launch
@@ -397,7 +398,8 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
         const bool overlap = prev >= 0 && prev != i && sg.pc_count == 0 && sg.kind[which] <= kPassRow;
         const bool in_line = (segs.size() > 1 || beside) && sg.kind[which] <= kPassRow;
         const int kind = in_line ? sg.kind[which] + kPassColLine : sg.kind[which];
-        PassArgs a{slots, items + sg.first, sg.count, nullptr, k, tw, which == 0 ? 1 : 0, overlap, beside};
+        PassArgs a{slots, items + sg.first, sg.count, nullptr, k, tw, which == 0 ? 1 : 0, overlap,
+                   beside && !idle, beside && idle};
         SP_CUDA_TRY(launch_pass(sg.N, sg.E, kind, sg.grid[which], st, a));
         prev = i;
       }
@@ -410,7 +412,8 @@ static int launch_line(const std::vector<Segment>& segs, const Slot* slots, cons
 // beside it on auxiliary streams, or after it where there are none.
 struct Lines {
   std::vector<std::vector<Segment>> line;
-  bool beside;  // the lines' passes know of one another (PassArgs.late, LINE kernels)
+  bool beside;  // the lines' passes know of one another (LINE kernels)
+  bool idle;    // all sizes together take no more than one round of the SMs
 };
 
 // The sizes whose passes take more than one round of the SMs share one line of
@@ -464,7 +467,7 @@ struct Lines {
 // 2 x 1024^2 983 / 903; 30 x 256^2 + 5 x 512^2 893 / 897.
 constexpr double kLineRounds = 90;
 static Lines lines_of(const std::vector<Segment>& segs, bool concurrent, bool capped) {
-  if (segs.size() == 1) return {{segs}, false};
+  if (segs.size() == 1) return {{segs}, false, false};
   double work = 0, rounds = 0;
   for (const Segment& sg : segs) {
     work += sg.work;
@@ -483,7 +486,7 @@ static Lines lines_of(const std::vector<Segment>& segs, bool concurrent, bool ca
     large += sg.N > 512;
   }
   const bool share = !concurrent || (large > 0 && (n > 2 || small == 0));
-  Lines r{std::vector<std::vector<Segment>>(1), false};
+  Lines r{std::vector<std::vector<Segment>>(1), false, rounds <= 1.0};
   for (const Segment& sg : segs)
     if (share && fits(sg)) r.line[0].push_back(sg);
   for (const Segment& sg : segs) {
@@ -503,7 +506,7 @@ static int launch_ticks(const Lines& lines, const Slot* slots, const Item* items
   const int n_aux = (int)lines.line.size() - 1;
   if (P == nullptr || n_aux == 0) {
     for (const auto& line : lines.line) {
-      const int rc = launch_line(line, slots, items, jobs, tw, lines.beside, st);
+      const int rc = launch_line(line, slots, items, jobs, tw, lines.beside, lines.idle, st);
       if (rc != SP_OK) return rc;
     }
     return SP_OK;
@@ -519,9 +522,10 @@ static int launch_ticks(const Lines& lines, const Slot* slots, const Item* items
     }
     forked = i + 1;
     if (rc == SP_OK)
-      rc = launch_line(lines.line[i + 1], slots, items, jobs, tw, lines.beside, P->streams[i]);
+      rc = launch_line(lines.line[i + 1], slots, items, jobs, tw, lines.beside, lines.idle, P->streams[i]);
   }
-  if (rc == SP_OK) rc = launch_line(lines.line[0], slots, items, jobs, tw, lines.beside, st);
+  if (rc == SP_OK)
+    rc = launch_line(lines.line[0], slots, items, jobs, tw, lines.beside, lines.idle, st);
   for (int i = 0; i < forked; ++i) {
     const cudaError_t e1 = cudaEventRecord(P->events[1 + i], P->streams[i]);
     const cudaError_t e2 = cudaStreamWaitEvent(st, P->events[1 + i], 0);
@@ -596,6 +600,9 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
   std::vector<int> ticks(n_groups, 0);
   int sms = 1;
   for (int g = 0; g < n_groups; ++g) {
+    bool side_by_side = false;  // other sizes run beside each one
+    for (int i = gstart[g]; concurrent && i < gstart[g + 1]; ++i)
+      side_by_side |= trials[i].n != trials[gstart[g]].n;
     for (int N = kMinN; N <= kMaxN; N *= 2) {
       const int E = chosen_e(N, opts);
       const int L_items = N / lines_per_item(N, E);
@@ -622,7 +629,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
         else if (trials[i].init == SP_INIT_RANDOM_PHASE) sg.col_ticks = std::max(sg.col_ticks, 1);
       }
       for (int p = 0; p < 2; ++p) {
-        const bool small = use_small_ctas(N, E, count, sms);
+        const bool small = !side_by_side && use_small_ctas(N, E, count, sms);
         if (small) sg.kind[p] = p == 0 ? kPassColSmall : kPassRowSmall;
         int per_sm = occ[sg.kind[p]];
         // (the cap is in large CTAs)
@@ -750,7 +757,7 @@ int sp::engine_run(const sp_trial* trials, int n_trials, void* workspace_dev, si
     }
     GraphKey key{workspace_dev, dev, g, ticks[g], {}};
     // (by lines: how they are split also depends on the algorithms)
-    key.shape.push_back(lines.beside);
+    key.shape.push_back(lines.beside + 2 * lines.idle);
     for (const auto& line : lines.line) {
       key.shape.push_back((int)line.size());
       for (const Segment& sg : line)

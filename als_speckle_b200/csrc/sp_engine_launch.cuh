@@ -16,6 +16,7 @@ struct PassArgs {
   int reverse;  // walk the item list from its end
   int overlap;  // independent of the previous kernel of the stream (see chain_start)
   int late;     // let the next kernel in only at the last item
+  int early;    // ... or at entry, before the wait
 };
 
 // The waits of programmatic launches (see pdl_allow_next).  A kernel whose
@@ -32,8 +33,11 @@ struct PassArgs {
 // then on is what L2 holds.  With `late`, each CTA lets it in only when it begins its last item:
 // CTAs let in earlier hold SMs that a concurrent line of launches could use (20 x
 // 512^2 beside 12 x 256^2: 86 against 91 us per iteration; alone, earlier is better,
-// 4 x 2048^2 266 against 268).
-// LINE kernels know both flags; the others, for a size alone on the chip, wait
+// 4 x 2048^2 266 against 268).  With `early` it lets it in before its own wait, so
+// that two kernels stand by: where several lines leave most SMs idle, launches are
+// what they wait for (40 x 64^2 beside 3 x 256^2, 60 iterations: 915 us, 969 let in
+// after the wait).
+// LINE kernels know the flags; the others, for a size alone on the chip, wait
 // and let go at their start (the flags' code in the loop costs the 2048^2 passes
 // 2%).
 template <bool LINE>
@@ -42,6 +46,7 @@ __device__ __forceinline__ void chain_start(const PassArgs& a) {
     __threadfence();
     return;
   }
+  if (LINE && a.early) pdl_allow_next();
   pdl_wait_prev();
   if (!(LINE && a.late)) pdl_allow_next();
 }
@@ -353,7 +358,9 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
 // CTAs, small CTAs in brackets: 256^2 x 1 8.5 / 6.1 [64], x 2 8.6 / 7.4 [128],
 // x 4 8.7 / 8.5 [256], x 8 9.3 / 10.5 [512]; 512^2 x 1 12.8 / 11.2 [128], x 4
 // 16.1 / 17.4 [512]; 128^2 x 1 14.7 / 8.4 [8], x 36 15.5 / 12.1 [288]; 64^2 x
-// 40 11.9 / 9.4 [80].  At 1024^2 a trial is 128 items already, and at 512^2 with
+// 40 11.9 / 9.4 [80].  Sizes that run side by side keep the large CTAs: small ones
+// of one size take the other's SMs (30 x 128^2 beside 512^2, 60 iterations: 1340 us,
+// 1306 with large ones; 4 x 256^2 beside 2 x 1024^2 2266 and 2130).  At 1024^2 a trial is 128 items already, and at 512^2 with
 // E < 32 one trial is more small CTAs than the rule takes.
 constexpr int kSmallThreads = 64;
 __host__ __device__ constexpr bool has_small_ctas(int N, int E) {

@@ -93,3 +93,14 @@ def test_capped_sizes_run_side_by_side(mix, tmp_path):
     (((128, 4), (512, 5), (1024, 2)), [{128}, {512, 1024}])])
 def test_sizes_of_a_pair_share_a_line_when_they_fill_their_sms(mix, lines, tmp_path):
     _check(mix, lines, tmp_path)
+
+
+@pytest.mark.parametrize("mix", [((128, 30), (512, 1)), ((256, 4), (1024, 2)), ((128, 8), (256, 2), (512, 1))])
+def test_small_ctas_are_for_a_size_alone(mix, tmp_path):
+    """Sizes side by side run in the large CTAs (of 128 or 256 threads); alone the small
+    counts here run in 64-thread ones, with the same results."""
+    for e in _check(mix, [{N} for N, _ in mix], tmp_path):
+        if "_pass" in e["name"]:
+            assert e["args"]["block"][0] > 64
+    alone = _check(mix[:1], [{mix[0][0]}], tmp_path)
+    assert {e["args"]["block"][0] for e in alone if "_pass" in e["name"]} == {64}
