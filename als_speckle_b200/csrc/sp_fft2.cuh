@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(kThreads) fft_cols_kernel(const float2* in,
 // the strips' transposition; with its stores in contiguous pieces 37), 71 us of
 // columns (instruction issue) and 6 us to add the partial sums up, against 435
 // us for embedding, two passes over the planes and an accumulation; columns
-// interleaved in a CTA, with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 53 us (rows
-// 14, columns 32, sums 5), from 128 us.  Radix 32 (two stages at 512) made the
+// interleaved in a CTA, with block barriers, took 128 us.  37 frames of 173 x 181, RFTF: 55 us (rows
+// 14, columns 32, sums 6), from 137 us.  Radix 32 (two stages at 512) made the
 // columns 65 us but changed the transforms' rounding.
 // ---------------------------------------------------------------------------
 struct EmbedArgs {
