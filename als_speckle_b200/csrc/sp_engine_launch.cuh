@@ -30,13 +30,14 @@ struct PassArgs {
 // through L1, which may still hold the lines that an earlier tick's pass read
 // there.  So an early start makes a device-scope fence first, which drops them;
 // nothing that runs beside the kernel writes these planes, so what is read from
-// then on is what L2 holds.  With `late`, each CTA lets it in only when it begins its last item:
-// CTAs let in earlier hold SMs that a concurrent line of launches could use (20 x
-// 512^2 beside 12 x 256^2: 86 against 91 us per iteration; alone, earlier is better,
-// 4 x 2048^2 266 against 268).  With `early` it lets it in before its own wait, so
-// that two kernels stand by: where several lines leave most SMs idle, launches are
-// what they wait for (40 x 64^2 beside 3 x 256^2, 60 iterations: 915 us, 969 let in
-// after the wait).
+// then on is what L2 holds.  With `late`, each CTA lets the next kernel in only
+// when it begins its last item: CTAs let in earlier hold SMs that a concurrent line
+// of launches could use (20 x 512^2 beside 12 x 256^2: 86 against 91 us per
+// iteration; alone, earlier is better, 4 x 2048^2 266 against 268).  With `early`
+// (lines of one size, which never set `overlap`) it lets it in before its own wait,
+// so that two kernels stand by: where several lines leave most SMs idle, launches
+// are what they wait for (40 x 64^2 beside 3 x 256^2, 60 iterations: 915 us, 969
+// let in after the wait).
 // LINE kernels know the flags; the others, for a size alone on the chip, wait
 // and let go at their start (the flags' code in the loop costs the 2048^2 passes
 // 2%).
@@ -351,17 +352,18 @@ __global__ void __launch_bounds__(kColSbThreads, 2) col_pass_sb_kernel(PassArgs 
 // Lone trials and small batches: when the items of kThreads-thread CTAs are
 // too few for the chip (a 256^2 trial is 16 of them at E = 16, on 16 of 148
 // SMs), both passes run in kSmallThreads-thread CTAs on quarter items (half items at
-// 64^2 with E = 32) instead (the same kernels, so bitwise the same results): a lone pass is bound by its
-// warps' own instruction chains, which run faster with 2 warps on an SM than
-// with 8.  Taken up to two small CTAs per SM (one at 512^2, where two of them
+// 64^2 with E = 32) instead (the same kernels, so bitwise the same results): a lone
+// pass is bound by its warps' own instruction chains, which run faster with 2 warps
+// on an SM than with 8.  Taken up to two small CTAs per SM (one at 512^2, where two of them
 // are as slow as a large one); measured, us per iteration in large / small
 // CTAs, small CTAs in brackets: 256^2 x 1 8.5 / 6.1 [64], x 2 8.6 / 7.4 [128],
 // x 4 8.7 / 8.5 [256], x 8 9.3 / 10.5 [512]; 512^2 x 1 12.8 / 11.2 [128], x 4
 // 16.1 / 17.4 [512]; 128^2 x 1 14.7 / 8.4 [8], x 36 15.5 / 12.1 [288]; 64^2 x
 // 40 11.9 / 9.4 [80].  Sizes that run side by side keep the large CTAs: small ones
 // of one size take the other's SMs (30 x 128^2 beside 512^2, 60 iterations: 1340 us,
-// 1306 with large ones; 4 x 256^2 beside 2 x 1024^2 2266 and 2130).  At 1024^2 a trial is 128 items already, and at 512^2 with
-// E < 32 one trial is more small CTAs than the rule takes.
+// 1306 with large ones; 4 x 256^2 beside 2 x 1024^2 2266 and 2130).  At 1024^2 a
+// trial is 128 items already, and at 512^2 with E < 32 one trial is more small CTAs
+// than the rule takes.
 constexpr int kSmallThreads = 64;
 __host__ __device__ constexpr bool has_small_ctas(int N, int E) {
   return N >= 64 && (N < 512 || (N == 512 && E == 32)) && pass_split(N, E, kSmallThreads) > 1;
